@@ -17,41 +17,30 @@
  *
  * The communicator-based API creates a pool per communicator (cuMemCreate /
  * cudaMalloc at init) and the test harness dccl_emu_collective allocates the
- * pools of its virtual ranks on every call. This entry point instead keeps the
- * scratch the two-shot all-reduce kernel needs (flag words and the staging
- * slots the ranks push their shards into) in a device array that is part of
- * the library image.
+ * pools of its virtual ranks on every call. This entry point needs no scratch
+ * at all: the buffers are on one device, so one kernel reads every rank's
+ * element, folds and writes the result to every rank.
  *
  * What it computes: for r in [0, nranks): outputs[r][i] = op(inputs[0][i], ...,
- * inputs[nranks-1][i]), i in [0, count). Same kernel phases, flag protocol and
- * accumulation order as the two-shot variant of ncclAllReduce (push shards to
- * their owners, reduce, pull the result shards), with "ranks" being groups of
- * CTAs of one cooperative launch.
+ * inputs[nranks-1][i]), i in [0, count). Same accumulation order as the
+ * two-shot variant of ncclAllReduce: the vector is cut into nranks shards of
+ * whole 16-byte vectors, and the fold of shard j starts at rank j and goes on
+ * with the other ranks in ascending order.
  *
  * Limits and rules:
  *   - nranks 1..DCCL_NOALLOC_MAX_RANKS, count * element size <=
  *     DCCL_NOALLOC_MAX_BYTES per rank; larger requests are refused with
  *     DCCL_NOALLOC_TOO_LARGE and a message on stderr, nothing is launched.
- *   - The scratch array is DCCL_NOALLOC_SCRATCH_BYTES (about 3.2 MB). Every
- *     device context that loads the library holds it until the process exits.
- *   - All calls on a device share that one array. The call clears the flag and
- *     status words it depends on (a memset on `stream`, ordered before the
- *     kernel); the staging part keeps the previous call's bytes, which are
- *     always overwritten before they are read. Two calls that overlap on the
- *     GPU (different streams, no ordering between them) race on the array:
- *     order them, e.g. by using one stream.
- *   - The first call on each device looks up the device address of the array
- *     (cudaGetSymbolAddress, with that device current) and caches it. That
- *     first call should be made before any stream capture begins.
+ *   - One ordinary kernel launch on `stream`, no state between calls: calls on
+ *     different streams may overlap, and a call can be captured in a graph.
  *   - inputs / outputs are host arrays of nranks device pointers (read during
  *     the call, not kept). Element pointers must be aligned to the element
- *     size; 16-byte aligned pointers take the vector path. outputs[r] may
- *     equal inputs[r].
- *   - device_status, when not null, is a device int the kernel sets to 0 on
- *     success or to 1 if a wait between the CTA groups gave up (bounded wait,
- *     2 s); read it after synchronising the stream.
- *   - The launch is cooperative (nranks x 4 CTAs), so it needs a device that
- *     supports cooperative launches and that many CTAs resident at once.
+ *     size; buffers that all have the same distance to a 16-byte boundary take
+ *     the vector path. outputs[r] may equal inputs[r] (or another rank's
+ *     input); buffers that overlap only partly are not supported.
+ *   - device_status, when not null, is a device int the kernel sets to 0. (The
+ *     ranks no longer wait for one another, so there is no wait that could give
+ *     up.)
  *   - No cudaMalloc, cudaFree, cudaMallocAsync, cudaHostAlloc or allocating
  *     library routine is called, on any path.
  */
@@ -64,11 +53,6 @@ extern "C" {
 
 #define DCCL_NOALLOC_MAX_RANKS 8
 #define DCCL_NOALLOC_MAX_BYTES (256u * 1024u)
-/* per rank: 16 KB of flag words + (ranks + 1) staging slots of MAX_BYTES / ranks (worst case, two ranks:
- * 1.5 x MAX_BYTES) + rounding slack; plus one status page for the whole array */
-#define DCCL_NOALLOC_RANK_BYTES (16u * 1024u + DCCL_NOALLOC_MAX_BYTES + DCCL_NOALLOC_MAX_BYTES / 2u + 4096u)
-#define DCCL_NOALLOC_SCRATCH_BYTES (DCCL_NOALLOC_MAX_RANKS * DCCL_NOALLOC_RANK_BYTES + 4096u)
-
 #define DCCL_NOALLOC_OK 0
 #define DCCL_NOALLOC_BAD_ARGUMENT (-1)
 #define DCCL_NOALLOC_TOO_LARGE (-2)

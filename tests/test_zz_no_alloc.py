@@ -3,8 +3,8 @@
 Some callers of the library may not allocate device memory when they need a reduction: all of it
 may be handed out to a caching allocator or a KV-cache pool, or they sit on a path where the
 device-wide synchronisation of cudaMalloc is not acceptable. For them the library exports
-dccl_allreduce_one_device_noalloc, an all-reduce among buffers on one device whose scratch is a
-fixed array inside the library image. This test calls it through its exported C symbol, the way
+dccl_allreduce_one_device_noalloc, an all-reduce among buffers on one device that needs no scratch.
+This test calls it through its exported C symbol, the way
 such a caller would, twice in a row on the same stream, and compares every rank's output with
 what the allocating entry point (dccl_emu_collective, two-shot variant) returns for the same
 inputs, and with a fold of the inputs computed on the CPU in fp64 / int64 (the two kernels share
@@ -108,3 +108,44 @@ def test_requests_beyond_the_built_in_scratch_are_refused(dccl_lib, capfd):
     assert fn(9, 7, 0, 4, ptrs, ptrs, None, None) == -1                        # more ranks than the array holds
     assert fn(2, 7, 0, 0, ptrs, ptrs, None, None) == 0                         # nothing to do
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("n,name,op,count,off", [
+    (8, "float32", "sum", 1, 0),                       # one element: no vector at all
+    (3, "float32", "sum", 4 * 128 + 3, 0),             # one full CTA of vectors and a tail
+    (5, "bfloat16", "sum", 1003, 1),                   # head of 7, vectors that cross shard ends
+    (7, "float16", "avg", 40, 3),                      # shards of one vector
+    (4, "int8", "prod", 4097, 5),
+    (2, "float64", "sum", MAX_BYTES // 8, 1),          # the limit behind a head of one element
+    (8, "uint8", "max", MAX_BYTES, 0),
+])
+@pytest.mark.parametrize("form", ["apart", "in_place", "crossed", "uneven"])
+def test_one_pass_equals_the_two_shot_fold_bit_for_bit(dccl_lib, n, name, op, count, off, form):
+    """Heads, tails, shard ends inside a vector, outputs that are another rank's input, and buffers whose distances to a
+    16-byte boundary differ. The fold order is the two-shot kernel's, so results are compared as bits."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    np_dt = np.dtype(np.uint16) if name == "bfloat16" else np.dtype(name)
+    ins = [oracle.make_input(name, count, seed=50 + r) for r in range(n)]
+    want = _reference(dccl_lib, n, name, op, count, ins)
+    np_carrier = {1: np.uint8, 2: np.int16, 4: np.int32, 8: np.int64}[np_dt.itemsize]
+    carrier = {1: torch.uint8, 2: torch.int16, 4: torch.int32, 8: torch.int64}[np_dt.itemsize]
+    offs = [off + (r % 2 if form == "uneven" else 0) for r in range(n)]
+    d_in = []
+    for x, o in zip(ins, offs):
+        buf = torch.zeros(count + o, dtype=carrier, device="cuda")
+        buf[o:].copy_(torch.from_numpy(x.view(np_carrier).copy()))
+        d_in.append(buf[o:])
+    guard = [torch.full((count + off + 8,), 0x55, dtype=carrier, device="cuda") for _ in range(n)]
+    d_out = d_in if form == "in_place" else d_in[1:] + d_in[:1] if form == "crossed" else [g[off:off + count] for g in guard]
+    status = torch.full((1,), 7, dtype=torch.int32, device="cuda")
+    rc = _entry(dccl_lib)(n, DTYPE_NAMES.index(name), OPS[op], count, (ctypes.c_void_p * n)(*[t.data_ptr() for t in d_in]),
+                          (ctypes.c_void_p * n)(*[t.data_ptr() for t in d_out]), status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    for r in range(n):
+        assert np.array_equal(d_out[r].cpu().numpy().view(np_dt).view(np_carrier), want[r].view(np_carrier)), r
+    for g in guard:      # nothing before or behind the outputs
+        assert torch.all(g[:off] == 0x55) and torch.all(g[off + count:] == 0x55)
