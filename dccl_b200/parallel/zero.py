@@ -9,7 +9,7 @@ drop to 1/world per rank.
 
     params -> one flat buffer per dtype (padded to world x 16 bytes), ``p.data`` and ``p.grad`` are views
     step:    reduce_scatter(avg) flat_grad -> grad slice (fp32 copy when the parameters are 16-bit)
-             inner optimizer on the master slice (fp32)
+             inner optimizer on the master slice (fp32); AdamW runs as one kernel together with the casts on either side
              all_gather the updated slice (cast back) into the flat parameter buffer
 
 With ``comm.world == 1`` this is the inner optimizer on a flat buffer. CPU tensors use the host path, CUDA
@@ -17,7 +17,15 @@ tensors the device kernels on the current stream; on GPUs with NVSwitch multicas
 symmetric memory (``symmetric=True``), so that both collectives run zero-copy through the switch. Call
 ``close()`` before the communicator is finalized to give that memory back.
 """
+import math
+
 import torch
+import torch.optim.optimizer as _optimizer
+
+from .._lib import lib
+from ..comm import DcclError, dtype_of
+
+_FUSED_DTYPES = (torch.bfloat16, torch.float16, torch.float32)
 
 
 class ShardedOptimizer:
@@ -68,19 +76,75 @@ class ShardedOptimizer:
 
     def step(self):
         comm, n = self.comm, self.comm.world
-        for g in self.groups:
-            if n > 1:
+        if n > 1:
+            for g in self.groups:
                 comm.reduce_scatter(g["grad"], g["grad_slice"], op="avg")
-                g["master"].grad.copy_(g["grad_slice"])
-            else:
-                g["master"].grad.copy_(g["grad"])
-        self.inner.step()
-        for g in self.groups:
-            if n > 1:
-                g["out_slice"].copy_(g["master"].detach())
+        updates = self._adamw_updates()
+        if updates is not None:
+            for u in updates:
+                self._adamw(*u)
+        else:
+            for g in self.groups:
+                g["master"].grad.copy_(g["grad_slice"] if n > 1 else g["grad"])
+            self.inner.step()
+            for g in self.groups:
+                (g["out_slice"] if n > 1 else g["flat"]).copy_(g["master"].detach())
+        if n > 1:
+            for g in self.groups:
                 comm.all_gather(g["out_slice"], g["flat"])
-            else:
-                g["flat"].copy_(g["master"].detach())
+
+    def _adamw_updates(self):
+        """(group, options, state) of every slice when one kernel per slice can do what ``inner.step()`` and the casts around
+        it do: plain AdamW on CUDA, past its first step (which makes the state), with nothing hooked into the step that
+        would have to see the gradient before or the result in between. None: the general path, which also reports
+        whatever is wrong with the state."""
+        inner = self.inner
+        if type(inner) is not torch.optim.AdamW or torch.compiler.is_compiling():
+            return None
+        if (inner._optimizer_step_pre_hooks or inner._optimizer_step_post_hooks or _optimizer._global_optimizer_pre_hooks
+                or _optimizer._global_optimizer_post_hooks):
+            return None
+        # a learning-rate scheduler wraps the step of its optimizer to see that it ran; any other replacement has to run
+        step = inner.__dict__.get("step")
+        if step is not None and not (getattr(step, "_wrapped_by_lr_sched", False) and getattr(step, "__wrapped__", None) is type(inner).step):
+            return None
+        if len(inner.param_groups) != 1 or len(inner.param_groups[0]["params"]) != len(self.groups):
+            return None
+        o = inner.param_groups[0]
+        if o["amsgrad"] or o["maximize"] or o["capturable"] or o["differentiable"] or o["fused"] or not o.get("decoupled_weight_decay", True):
+            return None
+        if not all(isinstance(x, (int, float)) for x in (o["lr"], o["weight_decay"], o["eps"]) + tuple(o["betas"])):
+            return None
+        updates = []
+        for g, p in zip(self.groups, o["params"]):
+            st = inner.state.get(p)
+            if p is not g["master"] or not p.is_cuda or not st or g["grad"].dtype not in _FUSED_DTYPES:
+                return None
+            if not torch.is_tensor(st.get("step")) or st["step"].is_cuda:
+                return None
+            for t in (p, p.grad, st.get("exp_avg"), st.get("exp_avg_sq")):
+                if t is None or type(t) not in (torch.Tensor, torch.nn.Parameter) or t.dtype != torch.float32 or t.device != p.device \
+                        or t.numel() != g["per"] or not t.is_contiguous():
+                    return None
+            updates.append((g, o, st))
+        if torch.cuda.is_current_stream_capturing():
+            return None
+        if step is not None:
+            inner._opt_called = True
+        return updates
+
+    def _adamw(self, g, o, st):
+        p, n = g["master"], self.comm.world
+        grad, out = (g["grad_slice"], g["out_slice"]) if n > 1 else (g["grad"], g["flat"])
+        m, v = st["exp_avg"], st["exp_avg_sq"]
+        st["step"] += 1
+        t, (b1, b2) = st["step"].item(), o["betas"]
+        rc = lib().dccl_adamw_flat(p.device.index, dtype_of(grad), g["per"], p.data_ptr(), p.grad.data_ptr(), m.data_ptr(), v.data_ptr(),
+                                   grad.data_ptr(), out.data_ptr(), 1 - o["lr"] * o["weight_decay"], 1 - b1, b2, 1 - b2,
+                                   o["lr"] / (1 - b1 ** t), math.sqrt(1 - b2 ** t), o["eps"], torch.cuda.current_stream(p.device).cuda_stream)
+        if rc != 0:
+            raise DcclError(1, "AdamW update")
+        torch.autograd.graph.increment_version((p, p.grad, m, v, out))
 
     def close(self):
         """Give symmetric buffers back (collective). The parameters keep their values in ordinary memory."""

@@ -1,0 +1,100 @@
+"""The one-kernel AdamW update of dccl_b200.parallel.zero against the general path (torch's own optimizer and the casts
+around it), and which optimizers may take it."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from dccl_b200.parallel import zero  # noqa: E402
+
+
+class OneProcess:
+    """The collectives of a world whose other ranks hold the same gradients (world 1 or 2), on the current device."""
+
+    rank, has_multicast = 0, False
+
+    def __init__(self, world):
+        self.world = world
+
+    def reduce_scatter(self, send, recv, op="sum"):
+        recv.copy_(send[:recv.numel()])
+
+    def all_gather(self, send, recv):
+        recv[:send.numel()].copy_(send)
+
+
+def _make(world, dtype, sizes, general, device="cuda", cls=torch.optim.AdamW, **kw):
+    torch.manual_seed(3)
+    params = [torch.nn.Parameter(torch.randn(s).to(dtype).to(device)) for s in sizes]
+    opt = zero.ShardedOptimizer(params, OneProcess(world), cls, symmetric=False, **dict(dict(lr=1e-2, betas=(0.9, 0.95), weight_decay=0.1), **kw))
+    if general:
+        opt.inner.register_step_pre_hook(lambda *a: None)      # anything hooked into the step keeps the general path
+    return opt
+
+
+def _train(opt, steps, scheduler=False):
+    sched = torch.optim.lr_scheduler.LambdaLR(opt.inner, lambda t: 0.5 ** t) if scheduler else None
+    for s in range(steps):
+        for i, g in enumerate(opt.groups):
+            gen = torch.Generator().manual_seed(100 * s + i)
+            g["grad"].copy_(torch.randn(g["grad"].numel(), generator=gen) * 10.0 ** (s - 2))
+        opt.step()
+        if sched:
+            sched.step()
+    return opt
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("world", [1, 2])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("sizes", [[3], [2048, 1], [2049 * 5, 7]])           # below one vector, one CTA, several and a tail
+@pytest.mark.parametrize("kw", [{}, {"betas": (0.0, 0.5), "weight_decay": 0.0}, {"betas": (0.4, 0.999), "scheduler": True}])
+def test_one_kernel_update_matches_the_general_path(dccl_lib, world, dtype, sizes, kw):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    kw, steps = dict(kw), 4
+    scheduler = kw.pop("scheduler", False)
+    a, b = (_train(_make(world, dtype, sizes, general, **kw), steps, scheduler) for general in (False, True))
+    assert a._adamw_updates() is not None and b._adamw_updates() is None
+    ga, gb = a.groups[0], b.groups[0]
+    sa, sb = a.inner.state[ga["master"]], b.inner.state[gb["master"]]
+    u = 2.0 ** -23
+    assert float(sa["step"]) == float(sb["step"]) == steps
+    assert torch.equal(ga["master"].grad, gb["master"].grad)
+    # every step rounds each moment a few times, relative to the gradients it mixes (up to 10 x 4 sigma, and their squares)
+    torch.testing.assert_close(sa["exp_avg"], sb["exp_avg"], rtol=4 * steps * u, atol=4 * steps * u * 50)
+    torch.testing.assert_close(sa["exp_avg_sq"], sb["exp_avg_sq"], rtol=4 * steps * u, atol=1e-30)
+    # the update is at most lr x |m| / sqrt(v) <= lr / sqrt(1 - beta2) off by such a rounding per step
+    lr, b2 = 1e-2, kw.get("betas", (0.9, 0.95))[1]
+    torch.testing.assert_close(ga["master"], gb["master"], rtol=steps * u, atol=16 * steps * u * lr / (1 - b2) ** 0.5)
+    ulp = {torch.float32: steps * u, torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -10}[dtype]
+    torch.testing.assert_close(ga["flat"].float(), gb["flat"].float(), rtol=ulp, atol=16 * steps * u * lr / (1 - b2) ** 0.5)
+
+
+@pytest.mark.gpu
+def test_state_that_is_not_aligned_takes_the_elementwise_loop(dccl_lib):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    a, b = (_train(_make(1, torch.bfloat16, [1000], general), 1) for general in (False, True))
+    st = a.inner.state[a.groups[0]["master"]]
+    for k in ("exp_avg", "exp_avg_sq"):                    # as after loading state that lies inside a larger buffer
+        buf = torch.zeros(st[k].numel() + 1, device="cuda")
+        buf[1:].copy_(st[k])
+        st[k] = buf[1:]
+    assert a._adamw_updates() is not None
+    a, b = _train(a, 2), _train(b, 2)
+    torch.testing.assert_close(a.groups[0]["master"], b.groups[0]["master"], rtol=3 * 2.0 ** -23, atol=1e-7)
+
+
+@pytest.mark.parametrize("kw,cls", [({"amsgrad": True}, torch.optim.AdamW), ({"maximize": True}, torch.optim.AdamW), ({}, torch.optim.Adam),
+                                    ({"lr": torch.tensor(1e-2)}, torch.optim.AdamW), ({}, torch.optim.SGD), ({}, torch.optim.AdamW)])
+def test_everything_else_stays_on_the_general_path(kw, cls):
+    """Options the kernel does not implement, other optimizers, and host tensors."""
+    opts = dict(kw)
+    if cls is torch.optim.SGD:
+        params = [torch.nn.Parameter(torch.randn(5))]
+        opt = zero.ShardedOptimizer(params, OneProcess(1), cls, symmetric=False, lr=0.1)
+    else:
+        opt = _make(1, torch.float32, [5], False, device="cpu", cls=cls, **opts)
+    before = opt.groups[0]["flat"].clone()
+    _train(opt, 2)
+    assert opt._adamw_updates() is None and not torch.equal(before, opt.groups[0]["flat"])
