@@ -19,13 +19,72 @@ static int sm_count() {
     return g_sm_count;
 }
 
-__global__ void __launch_bounds__(512) k_local_copy(char* __restrict__ dst, const char* __restrict__ src, size_t bytes) {
-    // each CTA takes one contiguous, 16-byte aligned piece
-    const size_t per = ((bytes + gridDim.x - 1) / gridDim.x + 15) / 16 * 16;
-    const size_t lo = per * blockIdx.x;
-    if (lo >= bytes) return;
-    const size_t n = bytes - lo < per ? bytes - lo : per;
-    copy_bytes(dst + lo, src + lo, n);
+/** Bytes k .. k+15 of the 32 bytes (a, b); k is the same for all threads of a launch. */
+__device__ __forceinline__ uint4 window16(uint4 a, uint4 b, unsigned k) {
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t x[6], y[5];
+#pragma unroll
+    for (int j = 0; j < 6; j++) x[j] = k & 8 ? w[j + 2] : w[j];
+#pragma unroll
+    for (int j = 0; j < 5; j++) y[j] = k & 4 ? x[j + 1] : x[j];
+    const unsigned r = (k & 3) * 8;
+    return make_uint4(__funnelshift_r(y[0], y[1], r), __funnelshift_r(y[1], y[2], r), __funnelshift_r(y[2], y[3], r), __funnelshift_r(y[3], y[4], r));
+}
+
+/** The 16 bytes at `p`, which lies k bytes behind a 16-byte boundary: one aligned vector, or a window over two. */
+__device__ __forceinline__ uint4 load16(const char* p, unsigned k) {
+    const uint4* q = reinterpret_cast<const uint4*>(p - k);
+    const uint4 a = q[0];
+    return k == 0 ? a : window16(a, q[1], k);
+}
+
+/**
+ * How a range is cut so that every store is a whole, aligned 16-byte vector whatever the two pointers are: `head` bytes up
+ * to the destination's first boundary, `nv` vectors, the rest. The source then lies `shift` bytes behind a boundary for all
+ * vectors alike. A source vector is read through the two aligned ones it lies in, so with a shift one vector more goes to
+ * the head where its first aligned one would begin before the source, and to the rest where its second one would end
+ * behind it: nothing outside the buffers is read.
+ */
+struct Cut {
+    size_t head, nv, rest;
+    unsigned shift;
+};
+
+static Cut cut_range(const void* dst, const void* src, size_t bytes) {
+    Cut c;
+    c.head = (16 - (reinterpret_cast<uintptr_t>(dst) & 15u)) & 15u;
+    c.shift = (unsigned)((reinterpret_cast<uintptr_t>(src) + c.head) & 15u);
+    if (c.head < c.shift) c.head += 16;
+    if (c.head > bytes) c.head = bytes;
+    c.nv = (bytes - c.head + c.shift) / 16;
+    if (c.shift && c.nv) c.nv--;
+    c.rest = bytes - c.head - c.nv * 16;
+    return c;
+}
+
+/**
+ * HBM bounds a large copy, launch and latency a small one. Every thread moves two vectors and the CTAs follow each other
+ * through memory, so that all SMs work in one window of a few MB: 1 GiB takes 312 us (6.9 TB/s of reads and writes) where
+ * two resident CTAs per SM, each on a contiguous piece of its own, took 363 us (296 places of memory open at once). The
+ * same shape is within 1 % of the best from 64 KB to 1 GiB (one to four vectors, 256 to 1024 threads, 16- and 32-byte
+ * accesses were tried), so there is one. Pointers with different distances to a 16-byte boundary cost a second load, which
+ * the L1 cache serves, and a few selects: 26 MB of bf16 from a source 6 bytes off take 12.3 us where a loop over single bytes
+ * took 88.2 us.
+ */
+constexpr int kCopyThreads = 256, kCopyU = 2;
+__global__ void __launch_bounds__(kCopyThreads) k_local_copy(char* __restrict__ dst, const char* __restrict__ src, const __grid_constant__ Cut c) {
+    const size_t i0 = (size_t)blockIdx.x * (kCopyThreads * kCopyU) + threadIdx.x;
+    uint4 v[kCopyU];
+#pragma unroll
+    for (int u = 0; u < kCopyU; u++)
+        if (i0 + u * kCopyThreads < c.nv) v[u] = load16(src + c.head + (i0 + u * kCopyThreads) * 16, c.shift);
+#pragma unroll
+    for (int u = 0; u < kCopyU; u++)
+        if (i0 + u * kCopyThreads < c.nv) *reinterpret_cast<uint4*>(dst + c.head + (i0 + u * kCopyThreads) * 16) = v[u];
+    if (blockIdx.x == 0) {      // at most 31 bytes before and 47 behind the vectors
+        for (size_t j = threadIdx.x; j < c.head; j += kCopyThreads) dst[j] = src[j];
+        for (size_t j = c.head + c.nv * 16 + threadIdx.x; j < c.head + c.nv * 16 + c.rest; j += kCopyThreads) dst[j] = src[j];
+    }
 }
 
 /**
@@ -75,11 +134,9 @@ __global__ void __launch_bounds__(512) k_local_reduce(T* acc, const T* __restric
 
 cudaError_t launch_local_copy(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
     if (!bytes || dst == src) return cudaSuccess;
-    // one CTA per SM, two when the message is large enough to keep them busy
-    size_t want = (bytes + (64u << 10) - 1) / (64u << 10);
-    int grid = (int)(want < (size_t)(2 * sm_count()) ? want : (size_t)(2 * sm_count()));
-    if (grid < 1) grid = 1;
-    k_local_copy<<<grid, 512, 0, stream>>>((char*)dst, (const char*)src, bytes);
+    const Cut c = cut_range(dst, src, bytes);
+    const size_t per = (size_t)kCopyThreads * kCopyU, grid = (c.nv + per - 1) / per;
+    k_local_copy<<<(unsigned)(grid ? grid : 1), kCopyThreads, 0, stream>>>((char*)dst, (const char*)src, c);
     return cudaGetLastError();
 }
 
