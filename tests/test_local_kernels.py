@@ -1,4 +1,4 @@
-"""The one-rank copy on device buffers at every distance from a 16-byte boundary, at lengths around
+"""The one-rank copy and the pairwise fold on device buffers at every distance from a 16-byte boundary, at lengths around
 the vector and CTA sizes: results are exact, and nothing around the destination is touched."""
 import os
 
@@ -7,6 +7,7 @@ import pytest
 torch = pytest.importorskip("torch")
 
 from dccl_b200 import Communicator  # noqa: E402
+from dccl_b200.comm import OPS, dtype_of  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -35,3 +36,45 @@ def test_copy_at_every_pair_of_offsets(comm, nbytes):
             want = torch.full_like(dst, 0xAB)
             want[do:do + nbytes] = src[so:so + nbytes]
             assert torch.equal(dst, want), (nbytes, so, do)
+
+
+@pytest.mark.parametrize("dtype", [torch.int8, torch.uint8, torch.int32, torch.int64, torch.float16, torch.bfloat16, torch.float32, torch.float64])
+@pytest.mark.parametrize("op", ["sum", "prod", "max", "min"])
+def test_fold_at_every_pair_of_offsets(dccl_lib, dtype, op):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    ve = 16 // torch.empty((), dtype=dtype).element_size()
+    stream = torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    for count in (1, 3 * ve + 1, 512 * ve, 512 * ve + ve + 3):
+        x = torch.randint(0, 12, (count + ve,), device="cuda", generator=gen).to(dtype)
+        a = torch.randint(0, 12, (count + ve,), device="cuda", generator=gen).to(dtype)      # products stay in the 8-bit range
+        if dtype.is_floating_point:
+            x += torch.rand(count + ve, device="cuda", generator=gen).to(dtype)
+            x[0], x[count // 2], a[count // 3] = float("inf"), float("nan"), float("-inf")
+        for ao in sorted({0, 1, ve // 2, ve - 1}):
+            for xo in sorted({0, 1, ve // 2, ve - 1}):
+                acc = a.clone()
+                rc = dccl_lib.dccl_local_reduce_device(acc[ao:].data_ptr(), x[xo:].data_ptr(), count, dtype_of(acc), OPS[op], stream)
+                assert rc == 0
+                p, q = a[ao:ao + count], x[xo:xo + count]
+                # 16-bit types: fp32 and one rounding, which is what torch's own operators do; a NaN loses to a number in max / min
+                if dtype.is_floating_point and op in ("max", "min"):
+                    r = torch.fmax(p, q) if op == "max" else torch.fmin(p, q)
+                else:
+                    r = {"sum": torch.add, "prod": torch.mul, "max": torch.maximum, "min": torch.minimum}[op](p, q)
+                want = a.clone()
+                want[ao:ao + count] = r
+                assert torch.equal(torch.nan_to_num(acc), torch.nan_to_num(want)) and torch.equal(acc.isnan(), want.isnan()), (count, ao, xo)
+
+
+def test_fold_into_itself_and_pointers_between_elements(dccl_lib):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    stream = torch.cuda.current_stream().cuda_stream
+    a = torch.arange(5003, dtype=torch.float32, device="cuda")[3:]
+    want = a + a
+    assert dccl_lib.dccl_local_reduce_device(a.data_ptr(), a.data_ptr(), a.numel(), dtype_of(a), OPS["sum"], stream) == 0
+    assert torch.equal(a, want)
+    assert dccl_lib.dccl_local_reduce_device(a.data_ptr() + 2, a.data_ptr(), 8, dtype_of(a), OPS["sum"], stream) != 0
+    assert torch.equal(a, want)
