@@ -3,6 +3,7 @@
  * between the reduce-scatter and the all-gather of dccl_b200/parallel/zero.py. Masters and moments are fp32; the gradient
  * arrives and the updated parameters leave in the parameters' own type.
  */
+#include "launch_early.cuh"
 #include "../device/reduce_ops.cuh"
 #include <cstdint>
 #include <cstdio>
@@ -40,11 +41,12 @@ __device__ __forceinline__ void adamw_element(const AdamWArgs& a, float g, float
 /**
  * 32 bytes per 16-bit parameter (gradient in, its fp32 copy out, master and moments both ways, parameter out), no reuse:
  * HBM bounds it. One pass instead of the fourteen of the elementwise form, which reads and writes every fp32 array three to
- * six times: 44 M bf16 parameters take 211 us instead of 991 us (6.7 TB/s). Every thread has two 16-byte accesses
+ * six times: 44 M bf16 parameters take 209 us instead of 991 us (6.7 TB/s). Every thread has two 16-byte accesses
  * of each array in flight; the arithmetic (two divisions, one square root) hides behind them.
  */
 template <typename T>
 __global__ void __launch_bounds__(kAdamWThreads) k_adamw(const __grid_constant__ AdamWArgs a, bool vec) {
+    wait_for_stream();
     using F = Pack<float, kAdamWN>;
     using P = Pack<T, kAdamWN>;
     const T* grad = reinterpret_cast<const T*>(a.grad);
@@ -111,14 +113,15 @@ extern "C" int dccl_adamw_flat(int device, int dtype, size_t n, void* master, vo
     bool vec = low % 16 == 0 && half % (dtype == 7 ? 16 : 8) == 0;
     const size_t per = (size_t)kAdamWThreads * kAdamWN * kAdamWU;
     const size_t blocks = (n + per - 1) / per;
-    const dim3 grid((unsigned)(blocks < 0x7fffffffu ? blocks : 0x7fffffffu)), block(kAdamWThreads);
-    if (grid.x < blocks) vec = false;
+    const unsigned grid = (unsigned)(blocks < 0x7fffffffu ? blocks : 0x7fffffffu);
+    if (grid < blocks) vec = false;
     int prev = -1;
     cudaGetDevice(&prev);
     cudaError_t e = prev != device ? cudaSetDevice(device) : cudaSuccess;
-    void* params[] = {&a, &vec};
-    const void* kernel = dtype == 6 ? (const void*)k_adamw<__half> : dtype == 7 ? (const void*)k_adamw<float> : dtype == 9 ? (const void*)k_adamw<__nv_bfloat16> : nullptr;
-    if (e == cudaSuccess) e = kernel ? cudaLaunchKernel(kernel, grid, block, params, 0, (cudaStream_t)stream_v) : cudaErrorInvalidValue;
+    cudaStream_t stream = (cudaStream_t)stream_v;
+    if (e == cudaSuccess)
+        e = dtype == 6 ? launch_early(k_adamw<__half>, grid, kAdamWThreads, stream, a, vec) : dtype == 7 ? launch_early(k_adamw<float>, grid, kAdamWThreads, stream, a, vec)
+            : dtype == 9 ? launch_early(k_adamw<__nv_bfloat16>, grid, kAdamWThreads, stream, a, vec) : cudaErrorInvalidValue;
     if (prev != device && prev >= 0) cudaSetDevice(prev);
     if (e == cudaSuccess) return 0;
     fprintf(stderr, "dccl_adamw_flat: %s\n", cudaGetErrorString(e));

@@ -3,6 +3,7 @@
  * only kernel, reference src/core/reduce.cu:9-38, as a vectorised, operator-
  * templated grid), and the bounded-wait self test.
  */
+#include "launch_early.cuh"
 #include "kernels.hpp"
 #include "../device/reduce_ops.cuh"
 
@@ -57,11 +58,12 @@ static Cut cut_range(const void* dst, const void* src, size_t bytes) {
  * two resident CTAs per SM, each on a contiguous piece of its own, took 363 us (296 places of memory open at once). The
  * same shape is within 1 % of the best from 64 KB to 1 GiB (one to four vectors, 256 to 1024 threads, 16- and 32-byte
  * accesses were tried), so there is one. Pointers with different distances to a 16-byte boundary cost a second load, which
- * the L1 cache serves, and a few selects: 26 MB of bf16 from a source 6 bytes off take 12.3 us where a loop over single bytes
+ * the L1 cache serves, and a few selects: 26 MB of bf16 from a source 6 bytes off take 9.9 us where a loop over single bytes
  * took 88.2 us.
  */
 constexpr int kCopyThreads = 256, kCopyU = 2;
 __global__ void __launch_bounds__(kCopyThreads) k_local_copy(char* __restrict__ dst, const char* __restrict__ src, const __grid_constant__ Cut c) {
+    wait_for_stream();
     const size_t i0 = (size_t)blockIdx.x * (kCopyThreads * kCopyU) + threadIdx.x;
     uint4 v[kCopyU];
 #pragma unroll
@@ -78,16 +80,17 @@ __global__ void __launch_bounds__(kCopyThreads) k_local_copy(char* __restrict__ 
 
 /**
  * acc[i] = op(acc[i], in[i]): three streams of HBM traffic and nothing else. One vector of each operand per thread, the
- * CTAs following each other through memory as in the copy: 1 GiB fp32 takes 448 us (7.2 TB/s), 25 MiB bf16 14.4 us and
- * 1 MiB 4.3 us (the host's cost of the call), where two resident CTAs per SM with eight vectors in flight per thread, each
+ * CTAs following each other through memory as in the copy: 1 GiB fp32 takes 448 us (7.2 TB/s), 25 MiB bf16 12.7 us and
+ * 1 MiB 3.6 us (the host's cost of the call), where two resident CTAs per SM with eight vectors in flight per thread, each
  * CTA on a piece of at least 64 KB, took 520, 16.4 and 5.1 us. Operands at different distances from a 16-byte boundary
- * read `in` through a window as the copy does: 12 MB of fp16 24.6 -> 6.2 us (before: one element per access). The elements outside the vectors get threads of their own behind the vectors' threads.
+ * read `in` through a window as the copy does: 12 MB of fp16 24.6 -> 4.4 us (before: one element per access). The elements outside the vectors get threads of their own behind the vectors' threads.
  */
 constexpr int kReduceThreads = 512;
 template <typename T, int OP>
 __global__ void __launch_bounds__(kReduceThreads) k_local_reduce(T* acc, const T* in, const __grid_constant__ Cut c) {
     using A = typename Traits<T>::Acc;
     constexpr int N = Vec16<T>::N;
+    wait_for_stream();
     const size_t t = (size_t)blockIdx.x * kReduceThreads + threadIdx.x;
     const size_t head = c.head / sizeof(T);
     if (t < c.nv) {
@@ -108,8 +111,7 @@ cudaError_t launch_local_copy(void* dst, const void* src, size_t bytes, cudaStre
     if (!bytes || dst == src) return cudaSuccess;
     const Cut c = cut_range(dst, src, bytes);
     const size_t per = (size_t)kCopyThreads * kCopyU, grid = (c.nv + per - 1) / per;
-    k_local_copy<<<(unsigned)(grid ? grid : 1), kCopyThreads, 0, stream>>>((char*)dst, (const char*)src, c);
-    return cudaGetLastError();
+    return launch_early(k_local_copy, (unsigned)(grid ? grid : 1), kCopyThreads, stream, (char*)dst, (const char*)src, c);
 }
 
 cudaError_t launch_local_reduce(void* acc, const void* in, size_t count, ncclDataType_t dt, ncclRedOp_t op, cudaStream_t stream) {
@@ -121,10 +123,11 @@ cudaError_t launch_local_reduce(void* acc, const void* in, size_t count, ncclDat
     const Cut c = cut_range(acc, in, count * es);
     const size_t threads = c.nv + (c.head + c.rest) / es;
     const unsigned grid = (unsigned)((threads + kReduceThreads - 1) / kReduceThreads);
-#define CALL(T, OP) k_local_reduce<T, OP><<<grid, kReduceThreads, 0, stream>>>((T*)acc, (const T*)in, c)
+    cudaError_t e = cudaErrorInvalidValue;
+#define CALL(T, OP) e = launch_early(k_local_reduce<T, OP>, grid, kReduceThreads, stream, (T*)acc, (const T*)in, c)
     DCCL_DISPATCH_TYPE_OP((int)dt, (int)op, CALL)
 #undef CALL
-    return cudaGetLastError();
+    return e;
 }
 
 /** Waits for a flag value that nothing ever writes; must return through the timeout path. */

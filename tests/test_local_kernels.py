@@ -78,3 +78,29 @@ def test_fold_into_itself_and_pointers_between_elements(dccl_lib):
     assert torch.equal(a, want)
     assert dccl_lib.dccl_local_reduce_device(a.data_ptr() + 2, a.data_ptr(), 8, dtype_of(a), OPS["sum"], stream) != 0
     assert torch.equal(a, want)
+
+
+def test_copy_and_fold_are_captured_and_replayed(comm, dccl_lib):
+    """Back to back on one stream, eager and from a graph: each call sees what the one before it wrote."""
+    n = (1 << 20) + 5
+    x = torch.arange(n, dtype=torch.float32, device="cuda")
+    a, b = torch.empty_like(x), torch.empty_like(x)
+
+    def chain():
+        stream = torch.cuda.current_stream().cuda_stream
+        comm.all_reduce(x, a)                                                                                   # a = x
+        assert dccl_lib.dccl_local_reduce_device(a.data_ptr(), x.data_ptr(), n, dtype_of(a), OPS["sum"], stream) == 0   # a = 2x
+        comm.all_reduce(a, b)
+        assert dccl_lib.dccl_local_reduce_device(b.data_ptr(), a.data_ptr(), n, dtype_of(a), OPS["sum"], stream) == 0   # b = 4x
+        x.add_(1.0)
+
+    for k in range(8):
+        chain()
+        assert torch.equal(b, 4 * (x - 1))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    for k in range(8):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(b, 4 * (x - 1)) and float(x[0]) == 16.0
