@@ -56,7 +56,7 @@ static Cut cut_range(const void* dst, const void* src, size_t bytes) {
  * HBM bounds a large copy, launch and latency a small one. Every thread moves two vectors and the CTAs follow each other
  * through memory, so that all SMs work in one window of a few MB: 1 GiB takes 312 us (6.9 TB/s of reads and writes) where
  * two resident CTAs per SM, each on a contiguous piece of its own, took 363 us (296 places of memory open at once). The
- * same shape is within 1 % of the best from 64 KB to 1 GiB (one to four vectors, 256 to 1024 threads, 16- and 32-byte
+ * same shape is within 3 % of the best from 64 KB to 1 GiB (one to four vectors, 256 to 1024 threads, 16- and 32-byte
  * accesses were tried), so there is one. Pointers with different distances to a 16-byte boundary cost a second load, which
  * the L1 cache serves, and a few selects: 26 MB of bf16 from a source 6 bytes off take 9.9 us where a loop over single bytes
  * took 88.2 us.

@@ -38,22 +38,36 @@ def _check(code, what):
         raise DcclError(code, what)
 
 
+_torch_module = None
+_torch_dtypes = {}
+
+
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        table = {torch.int8: INT8, torch.uint8: UINT8, torch.int32: INT32, torch.int64: INT64, torch.float16: FLOAT16,
+                 torch.float32: FLOAT32, torch.float64: FLOAT64, torch.bfloat16: BFLOAT16}
+        if hasattr(torch, "uint32"):
+            table[torch.uint32] = UINT32
+            table[torch.uint64] = UINT64
+        _torch_dtypes.update(table)
+        _torch_module = torch
+    return _torch_module
 
 
 def dtype_of(x):
     """ncclDataType_t value of a numpy array or torch tensor."""
     if isinstance(x, np.ndarray):
         return _NP_TO_DCCL[x.dtype]
-    torch = _torch()
-    table = {torch.int8: INT8, torch.uint8: UINT8, torch.int32: INT32, torch.int64: INT64, torch.float16: FLOAT16,
-             torch.float32: FLOAT32, torch.float64: FLOAT64, torch.bfloat16: BFLOAT16}
-    if hasattr(torch, "uint32"):
-        table[torch.uint32] = UINT32
-        table[torch.uint64] = UINT64
-    return table[x.dtype]
+    if not _torch_dtypes:
+        _torch()
+    return _torch_dtypes[x.dtype]
+
+
+def current_stream_handle(device):
+    """cudaStream_t of torch's current stream on device `device` (an index), without a Stream object around it."""
+    return _torch()._C._cuda_getCurrentRawStream(device)
 
 
 def _addr(x):
@@ -78,7 +92,7 @@ def _stream_of(x, stream):
     if isinstance(x, np.ndarray):
         return None
     if x.is_cuda:
-        return _torch().cuda.current_stream(x.device).cuda_stream
+        return current_stream_handle(x.get_device())
     return None
 
 

@@ -23,7 +23,7 @@ import torch
 import torch.optim.optimizer as _optimizer
 
 from .._lib import lib
-from ..comm import DcclError, dtype_of
+from ..comm import DcclError, current_stream_handle, dtype_of
 
 _FUSED_DTYPES = (torch.bfloat16, torch.float16, torch.float32)
 
@@ -113,18 +113,19 @@ class ShardedOptimizer:
         o = inner.param_groups[0]
         if o["amsgrad"] or o["maximize"] or o["capturable"] or o["differentiable"] or o["fused"] or not o.get("decoupled_weight_decay", True):
             return None
-        if not all(isinstance(x, (int, float)) for x in (o["lr"], o["weight_decay"], o["eps"]) + tuple(o["betas"])):
-            return None
+        for x in (o["lr"], o["weight_decay"], o["eps"], *o["betas"]):
+            if not isinstance(x, (int, float)):
+                return None
         updates = []
         for g, p in zip(self.groups, o["params"]):
             st = inner.state.get(p)
             if p is not g["master"] or not p.is_cuda or not st or g["grad"].dtype not in _FUSED_DTYPES:
                 return None
-            if not torch.is_tensor(st.get("step")) or st["step"].is_cuda:
+            step_count, device, per = st.get("step"), p.get_device(), g["per"]
+            if not isinstance(step_count, torch.Tensor) or step_count.is_cuda:
                 return None
             for t in (p, p.grad, st.get("exp_avg"), st.get("exp_avg_sq")):
-                if t is None or type(t) not in (torch.Tensor, torch.nn.Parameter) or t.dtype != torch.float32 or t.device != p.device \
-                        or t.numel() != g["per"] or not t.is_contiguous():
+                if type(t) is not torch.Tensor or t.dtype is not torch.float32 or t.get_device() != device or t.numel() != per or not t.is_contiguous():
                     return None
             updates.append((g, o, st))
         if torch.cuda.is_current_stream_capturing():
@@ -135,13 +136,14 @@ class ShardedOptimizer:
 
     def _adamw(self, g, o, st):
         p, n = g["master"], self.comm.world
+        device = p.get_device()
         grad, out = (g["grad_slice"], g["out_slice"]) if n > 1 else (g["grad"], g["flat"])
         m, v = st["exp_avg"], st["exp_avg_sq"]
-        st["step"] += 1
-        t, (b1, b2) = st["step"].item(), o["betas"]
-        rc = lib().dccl_adamw_flat(p.device.index, dtype_of(grad), g["per"], p.data_ptr(), p.grad.data_ptr(), m.data_ptr(), v.data_ptr(),
+        t, (b1, b2) = st["step"].item() + 1, o["betas"]
+        st["step"].fill_(t)
+        rc = lib().dccl_adamw_flat(device, dtype_of(grad), g["per"], p.data_ptr(), p.grad.data_ptr(), m.data_ptr(), v.data_ptr(),
                                    grad.data_ptr(), out.data_ptr(), 1 - o["lr"] * o["weight_decay"], 1 - b1, b2, 1 - b2,
-                                   o["lr"] / (1 - b1 ** t), math.sqrt(1 - b2 ** t), o["eps"], torch.cuda.current_stream(p.device).cuda_stream)
+                                   o["lr"] / (1 - b1 ** t), math.sqrt(1 - b2 ** t), o["eps"], current_stream_handle(device))
         if rc != 0:
             raise DcclError(1, "AdamW update")
         torch.autograd.graph.increment_version((p, p.grad, m, v, out))
