@@ -23,9 +23,8 @@ struct AdamWArgs {
     float eps;
 };
 
-constexpr int kAdamWThreads = 256;
+constexpr int kAdamWThreads = 128;
 constexpr int kAdamWN = 4;              // elements of one access: 16 bytes of fp32
-constexpr int kAdamWU = 2;              // accesses in flight per array and thread
 
 template <typename T, int N> struct alignas(sizeof(T) * N) Pack { T e[N]; };
 
@@ -41,8 +40,10 @@ __device__ __forceinline__ void adamw_element(const AdamWArgs& a, float g, float
 /**
  * 32 bytes per 16-bit parameter (gradient in, its fp32 copy out, master and moments both ways, parameter out), no reuse:
  * HBM bounds it. One pass instead of the fourteen of the elementwise form, which reads and writes every fp32 array three to
- * six times: 44 M bf16 parameters take 209 us instead of 991 us (6.7 TB/s). Every thread has two 16-byte accesses
- * of each array in flight; the arithmetic (two divisions, one square root) hides behind them.
+ * six times: 44 M bf16 parameters take 209 us instead of 991 us (6.7 TB/s). One 16-byte access of each
+ * fp32 array per thread and CTAs of 128; two accesses and CTAs of 256 took 0.3 % longer at 44 M and 1.7 % longer at 4 M
+ * parameters (128 to 1024 threads with one, two and four accesses were tried). The arithmetic (two divisions, one square
+ * root) hides behind the loads.
  */
 template <typename T>
 __global__ void __launch_bounds__(kAdamWThreads) k_adamw(const __grid_constant__ AdamWArgs a, bool vec) {
@@ -52,38 +53,22 @@ __global__ void __launch_bounds__(kAdamWThreads) k_adamw(const __grid_constant__
     const T* grad = reinterpret_cast<const T*>(a.grad);
     T* out = reinterpret_cast<T*>(a.out);
     if (vec) {
-        const size_t nv = a.n / kAdamWN;
-        const size_t base = (size_t)blockIdx.x * (kAdamWThreads * kAdamWU) + threadIdx.x;
-        P g[kAdamWU];
-        F p[kAdamWU], m[kAdamWU], v[kAdamWU];
+        const size_t i = (size_t)blockIdx.x * kAdamWThreads + threadIdx.x;
+        if (i < a.n / kAdamWN) {
+            const P g = reinterpret_cast<const P*>(grad)[i];
+            F p = reinterpret_cast<const F*>(a.master)[i], m = reinterpret_cast<const F*>(a.m)[i], v = reinterpret_cast<const F*>(a.v)[i], gf;
+            P o;
 #pragma unroll
-        for (int u = 0; u < kAdamWU; u++) {
-            const size_t i = base + (size_t)u * kAdamWThreads;
-            if (i < nv) {
-                g[u] = reinterpret_cast<const P*>(grad)[i];
-                p[u] = reinterpret_cast<const F*>(a.master)[i];
-                m[u] = reinterpret_cast<const F*>(a.m)[i];
-                v[u] = reinterpret_cast<const F*>(a.v)[i];
+            for (int e = 0; e < kAdamWN; e++) {
+                gf.e[e] = Traits<T>::up(g.e[e]);
+                adamw_element(a, gf.e[e], p.e[e], m.e[e], v.e[e]);
+                o.e[e] = Traits<T>::down(p.e[e]);
             }
-        }
-#pragma unroll
-        for (int u = 0; u < kAdamWU; u++) {
-            const size_t i = base + (size_t)u * kAdamWThreads;
-            if (i < nv) {
-                F gf;
-                P o;
-#pragma unroll
-                for (int e = 0; e < kAdamWN; e++) {
-                    gf.e[e] = Traits<T>::up(g[u].e[e]);
-                    adamw_element(a, gf.e[e], p[u].e[e], m[u].e[e], v[u].e[e]);
-                    o.e[e] = Traits<T>::down(p[u].e[e]);
-                }
-                reinterpret_cast<F*>(a.master_grad)[i] = gf;
-                reinterpret_cast<F*>(a.master)[i] = p[u];
-                reinterpret_cast<F*>(a.m)[i] = m[u];
-                reinterpret_cast<F*>(a.v)[i] = v[u];
-                reinterpret_cast<P*>(out)[i] = o;
-            }
+            reinterpret_cast<F*>(a.master_grad)[i] = gf;
+            reinterpret_cast<F*>(a.master)[i] = p;
+            reinterpret_cast<F*>(a.m)[i] = m;
+            reinterpret_cast<F*>(a.v)[i] = v;
+            reinterpret_cast<P*>(out)[i] = o;
         }
     }
     // arrays that are not aligned, or the last elements of an odd length
@@ -111,7 +96,7 @@ extern "C" int dccl_adamw_flat(int device, int dtype, size_t n, void* master, vo
     const uintptr_t low = (uintptr_t)master | (uintptr_t)master_grad | (uintptr_t)m | (uintptr_t)v;
     const uintptr_t half = (uintptr_t)grad | (uintptr_t)out;
     bool vec = low % 16 == 0 && half % (dtype == 7 ? 16 : 8) == 0;
-    const size_t per = (size_t)kAdamWThreads * kAdamWN * kAdamWU;
+    const size_t per = (size_t)kAdamWThreads * kAdamWN;
     const size_t blocks = (n + per - 1) / per;
     const unsigned grid = (unsigned)(blocks < 0x7fffffffu ? blocks : 0x7fffffffu);
     if (grid < blocks) vec = false;

@@ -85,6 +85,31 @@ def test_state_that_is_not_aligned_takes_the_elementwise_loop(dccl_lib):
     torch.testing.assert_close(a.groups[0]["master"], b.groups[0]["master"], rtol=3 * 2.0 ** -23, atol=1e-7)
 
 
+@pytest.mark.gpu
+def test_two_slices_changed_options_and_loaded_state(dccl_lib):
+    """One kernel per dtype; options changed between steps and state that went through state_dict are what the step uses."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+
+    def make(general):
+        torch.manual_seed(3)
+        params = [torch.nn.Parameter(torch.randn(s, device="cuda").to(d)) for s, d in ((1001, torch.bfloat16), (77, torch.float32), (30, torch.bfloat16))]
+        opt = zero.ShardedOptimizer(params, OneProcess(1), symmetric=False, lr=1e-2)
+        if general:
+            opt.inner.register_step_pre_hook(lambda *a: None)
+        return opt
+
+    a, b = _train(make(False), 2), _train(make(True), 2)
+    for opt in (a, b):
+        opt.inner.load_state_dict(opt.inner.state_dict())
+        opt.inner.param_groups[0].update(lr=3e-3, weight_decay=0.5, eps=1e-4)
+    assert len(a.groups) == 2 and a._adamw_updates() is not None
+    a, b = _train(a, 2), _train(b, 2)
+    for ga, gb in zip(a.groups, b.groups):
+        torch.testing.assert_close(ga["master"], gb["master"], rtol=4 * 2.0 ** -23, atol=1e-7)
+        assert float(a.inner.state[ga["master"]]["step"]) == 4
+
+
 @pytest.mark.parametrize("kw,cls", [({"amsgrad": True}, torch.optim.AdamW), ({"maximize": True}, torch.optim.AdamW), ({}, torch.optim.Adam),
                                     ({"lr": torch.tensor(1e-2)}, torch.optim.AdamW), ({}, torch.optim.SGD), ({}, torch.optim.AdamW)])
 def test_everything_else_stays_on_the_general_path(kw, cls):
