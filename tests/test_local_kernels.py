@@ -104,3 +104,24 @@ def test_copy_and_fold_are_captured_and_replayed(comm, dccl_lib):
         graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(b, 4 * (x - 1)) and float(x[0]) == 16.0
+
+
+def test_calls_wait_for_other_streams_and_for_copies_and_fills(comm, dccl_lib):
+    """An event of another stream, a copy or a fill between two calls is waited for like by any kernel."""
+    n = 1 << 20
+    x, y, a = (torch.zeros(n, device="cuda") for _ in range(3))
+    host = torch.empty(n, pin_memory=True)
+    side = torch.cuda.Stream()
+    here = torch.cuda.current_stream()
+    for k in range(1, 21):
+        comm.all_reduce(x, a)                       # a call right before, so that the next one could be set up early
+        side.wait_stream(here)
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(200000)
+            x.fill_(float(k))
+        here.wait_stream(side)
+        comm.all_reduce(x, y)                       # reads what the other stream has just written
+        host.fill_(float(k))
+        a.copy_(host, non_blocking=True)            # a copy, then a fold of its destination
+        assert dccl_lib.dccl_local_reduce_device(a.data_ptr(), y.data_ptr(), n, dtype_of(a), OPS["sum"], here.cuda_stream) == 0
+        assert torch.equal(a, torch.full_like(a, 2.0 * k)) and torch.equal(y, torch.full_like(y, float(k))), k
