@@ -26,8 +26,6 @@ struct AdamWArgs {
 constexpr int kAdamWThreads = 128;
 constexpr int kAdamWN = 4;              // elements of one access: 16 bytes of fp32
 
-template <typename T, int N> struct alignas(sizeof(T) * N) Pack { T e[N]; };
-
 /** Each operation rounds as torch's AdamW does one by one (moments as lerp and addcmul, true division and square root),
  *  except that a product feeding a sum is fused. */
 __device__ __forceinline__ void adamw_element(const AdamWArgs& a, float g, float& p, float& m, float& v) {

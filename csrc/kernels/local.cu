@@ -3,6 +3,7 @@
  * only kernel, reference src/core/reduce.cu:9-38, as a vectorised, operator-
  * templated grid), and the bounded-wait self test.
  */
+#include "byte_ops.cuh"
 #include "launch_early.cuh"
 #include "kernels.hpp"
 #include "../device/reduce_ops.cuh"
@@ -97,8 +98,11 @@ __global__ void __launch_bounds__(kReduceThreads) k_local_reduce(T* acc, const T
         T* p = acc + head + t * N;
         Vec16<T> x = ld_vec<T>(p), y;
         *reinterpret_cast<uint4*>(&y) = load16(reinterpret_cast<const char*>(in + head + t * N), c.shift);
+        if constexpr (kFoldsBytes<T, OP>) fold_bytes<T, OP>(x, y);
+        else {
 #pragma unroll
-        for (int e = 0; e < N; e++) x.e[e] = Traits<T>::down(op_apply<OP, A>(Traits<T>::up(x.e[e]), Traits<T>::up(y.e[e])));
+            for (int e = 0; e < N; e++) x.e[e] = Traits<T>::down(op_apply<OP, A>(Traits<T>::up(x.e[e]), Traits<T>::up(y.e[e])));
+        }
         st_vec<T>(p, x);
         return;
     }

@@ -149,3 +149,31 @@ def test_one_pass_equals_the_two_shot_fold_bit_for_bit(dccl_lib, n, name, op, co
         assert np.array_equal(d_out[r].cpu().numpy().view(np_dt).view(np_carrier), want[r].view(np_carrier)), r
     for g in guard:      # nothing before or behind the outputs
         assert torch.all(g[:off] == 0x55) and torch.all(g[off + count:] == 0x55)
+
+
+@pytest.mark.parametrize("name", ["int8", "uint8"])
+@pytest.mark.parametrize("op", ["sum", "avg", "max", "min", "prod"])
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 8])
+def test_bytes_of_the_whole_range(dccl_lib, name, op, n):
+    """Whole vectors of bytes fold four at a time and divide by multiplying: every value, wrapping sums, both signs."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    rng = np.random.default_rng(n)
+    count = 2048 + 5
+    ins = [rng.integers(0, 256, count).astype(np.uint8).view(name) for _ in range(n)]
+    ins[0][:256] = np.arange(256).astype(np.uint8).view(name)
+    for x in ins[1:]:
+        x[:256] = 0                                  # every value once, divided by n
+    want = oracle.fold(ins, op)
+    d_in = [torch.from_numpy(x.view(np.uint8).copy()).to("cuda") for x in ins]
+    d_out = [torch.empty_like(x) for x in d_in]
+    rc = _entry(dccl_lib)(n, DTYPE_NAMES.index(name), OPS[op], count, (ctypes.c_void_p * n)(*[t.data_ptr() for t in d_in]),
+                          (ctypes.c_void_p * n)(*[t.data_ptr() for t in d_out]), None, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    for t in d_out:
+        assert np.array_equal(t.cpu().numpy().view(name), want)
+    if n == 2:                                        # the pairwise fold of the same bytes (an average accumulates like a sum)
+        rc = dccl_lib.dccl_local_reduce_device(d_in[0].data_ptr(), d_in[1].data_ptr(), count, DTYPE_NAMES.index(name), OPS[op],
+                                               torch.cuda.current_stream().cuda_stream)
+        assert rc == 0 and np.array_equal(d_in[0].cpu().numpy().view(name), oracle.fold(ins, "sum" if op == "avg" else op))
