@@ -27,11 +27,12 @@ constexpr int kAdamWThreads = 128;
 constexpr int kAdamWN = 4;              // elements of one access: 16 bytes of fp32
 
 /** Each operation rounds as torch's AdamW does one by one (moments as lerp and addcmul, true division and square root),
- *  except that a product feeding a sum is fused. */
+ *  except that a product feeding a sum is fused. The square of the gradient comes first, so that it overflows where torch's
+ *  does: the element is then not updated any more. */
 __device__ __forceinline__ void adamw_element(const AdamWArgs& a, float g, float& p, float& m, float& v) {
     p *= a.decay;
     m = a.w1 < 0.5f ? fmaf(a.w1, g - m, m) : fmaf(-(1.0f - a.w1), g - m, g);
-    v = fmaf(a.w2 * g, g, a.b2 * v);
+    v = fmaf(a.w2, g * g, a.b2 * v);
     p = fmaf(-a.step, m / (sqrtf(v) / a.bc2_sqrt + a.eps), p);
 }
 

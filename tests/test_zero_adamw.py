@@ -86,6 +86,31 @@ def test_state_that_is_not_aligned_takes_the_elementwise_loop(dccl_lib):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kw", [{}, {"betas": (0.0, 0.0), "eps": 0.0}, {"betas": (0.6, 0.999)}])
+def test_infinities_nan_and_gradients_whose_squares_leave_the_range(dccl_lib, dtype, kw):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    vals = torch.tensor([float("inf"), float("-inf"), float("nan"), 2e19, -2e19, 1e20, 3e38, -3e38, 1.8e19, 1.9e19, 5e18, 1e-22, 1e-40, 0.0, 1.0], device="cuda")
+    outs = []
+    for general in (False, True):
+        opt = _make(1, dtype, [vals.numel()], general, **kw)
+        g = opt.groups[0]
+        for sign in (0.0, 1.0, -1.0, 1.0):           # a plain step first
+            g["grad"].zero_()
+            if sign:
+                g["grad"][:vals.numel()] = (sign * vals).to(dtype)
+            opt.step()
+        st = opt.inner.state[g["master"]]
+        outs.append([t.detach().clone() for t in (g["master"], g["flat"], st["exp_avg"], st["exp_avg_sq"])])
+    for x, y in zip(*outs):
+        assert torch.equal(x.isnan(), y.isnan()) and torch.equal(x.isinf(), y.isinf())
+        fine = y.isfinite()
+        # a few roundings per step, relative to gradients of both signs
+        torch.testing.assert_close(x[fine].float(), y[fine].float(), rtol=2.0 ** -7 if x.dtype == torch.bfloat16 else 1e-5, atol=1e-7)
+
+
+@pytest.mark.gpu
 def test_two_slices_changed_options_and_loaded_state(dccl_lib):
     """One kernel per dtype; options changed between steps and state that went through state_dict are what the step uses."""
     if not torch.cuda.is_available():
