@@ -84,7 +84,8 @@ __global__ void __launch_bounds__(kCopyThreads) k_local_copy(char* __restrict__ 
  * CTAs following each other through memory as in the copy: 1 GiB fp32 takes 448 us (7.2 TB/s), 25 MiB bf16 12.7 us and
  * 1 MiB 3.6 us (the host's cost of the call), where two resident CTAs per SM with eight vectors in flight per thread, each
  * CTA on a piece of at least 64 KB, took 520, 16.4 and 5.1 us. Operands at different distances from a 16-byte boundary
- * read `in` through a window as the copy does: 12 MB of fp16 24.6 -> 4.4 us (before: one element per access). The elements outside the vectors get threads of their own behind the vectors' threads.
+ * read `in` through a window as the copy does: 12 MB of fp16 24.6 -> 4.4 us (before: one element per access). The elements
+ * outside the vectors get threads of their own behind the vectors' threads.
  */
 constexpr int kReduceThreads = 512;
 template <typename T, int OP>

@@ -53,6 +53,9 @@ extern "C" {
 
 #define DCCL_NOALLOC_MAX_RANKS 8
 #define DCCL_NOALLOC_MAX_BYTES (256u * 1024u)
+/* device memory the library holds for this entry point: none */
+#define DCCL_NOALLOC_SCRATCH_BYTES 0u
+
 #define DCCL_NOALLOC_OK 0
 #define DCCL_NOALLOC_BAD_ARGUMENT (-1)
 #define DCCL_NOALLOC_TOO_LARGE (-2)
