@@ -177,3 +177,20 @@ def test_bytes_of_the_whole_range(dccl_lib, name, op, n):
         rc = dccl_lib.dccl_local_reduce_device(d_in[0].data_ptr(), d_in[1].data_ptr(), count, DTYPE_NAMES.index(name), OPS[op],
                                                torch.cuda.current_stream().cuda_stream)
         assert rc == 0 and np.array_equal(d_in[0].cpu().numpy().view(name), oracle.fold(ins, "sum" if op == "avg" else op))
+
+
+@pytest.mark.parametrize("name,count", [("float32", 1), ("bfloat16", 1003), ("float64", MAX_BYTES // 8)])
+@pytest.mark.parametrize("in_off,out_off", [(1, 1), (0, 1), (3, 6), (5, 5)])
+def test_one_rank_copies_from_and_to_any_address(dccl_lib, name, count, in_off, out_off):
+    """Addresses between two elements included: a copy has no elements."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    nbytes = count * np.dtype("uint16" if name == "bfloat16" else name).itemsize
+    src = torch.randint(0, 255, (nbytes + 16,), dtype=torch.uint8, device="cuda")
+    dst = torch.full((nbytes + 16,), 0xAB, dtype=torch.uint8, device="cuda")
+    want = dst.clone()
+    want[out_off:out_off + nbytes] = src[in_off:in_off + nbytes]
+    rc = _entry(dccl_lib)(1, DTYPE_NAMES.index(name), OPS["sum"], count, (ctypes.c_void_p * 1)(src.data_ptr() + in_off),
+                          (ctypes.c_void_p * 1)(dst.data_ptr() + out_off), None, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and torch.equal(dst, want)
