@@ -149,6 +149,12 @@ extern "C" int dccl_allreduce_one_device_noalloc(int nranks, int dtype, int op, 
         dtype = 1;
         es = 1;
     }
+    // everywhere else the kernel loads and stores elements
+    for (int r = 0; r < nranks; r++)
+        if ((((uintptr_t)inputs[r] | (uintptr_t)outputs[r]) & (es - 1)) != 0) {
+            fprintf(stderr, "dccl_allreduce_one_device_noalloc: buffer of rank %d lies between two elements of %zu bytes\n", r, es);
+            return DCCL_NOALLOC_BAD_ARGUMENT;
+        }
 
     NoAllocArgs a;
     a.nranks = nranks;
@@ -157,9 +163,9 @@ extern "C" int dccl_allreduce_one_device_noalloc(int nranks, int dtype, int op, 
     // shards as the two-shot all-reduce cuts them: whole 16-byte vectors
     const unsigned ve = (unsigned)(16 / es);
     a.per = (unsigned)((count + nranks - 1) / nranks + ve - 1) / ve * ve;
-    // 16-byte accesses when every buffer has the same distance to a 16-byte boundary (a multiple of the element size)
+    // 16-byte accesses when every buffer has the same distance to a 16-byte boundary
     const uintptr_t mis = (uintptr_t)inputs[0] & 15u;
-    bool vec = mis % es == 0;
+    bool vec = true;
     for (int r = 0; r < DCCL_NOALLOC_MAX_RANKS; r++) {
         a.in[r] = r < nranks ? inputs[r] : nullptr;
         a.out[r] = r < nranks ? outputs[r] : nullptr;

@@ -35,10 +35,11 @@
  *     different streams may overlap, and a call can be captured in a graph.
  *   - inputs / outputs are host arrays of nranks device pointers (read during
  *     the call, not kept). Element pointers must be aligned to the element
- *     size (with one rank, whose call is a copy, they need not be); buffers
- *     that all have the same distance to a 16-byte boundary take the vector
- *     path. outputs[r] may equal inputs[r] (or another rank's input); buffers
- *     that overlap only partly are not supported.
+ *     size, or the call is refused with DCCL_NOALLOC_BAD_ARGUMENT (with one
+ *     rank, whose call is a copy, they need not be); buffers that all have the
+ *     same distance to a 16-byte boundary take the vector path. outputs[r] may
+ *     equal inputs[r] (or another rank's input); buffers that overlap only
+ *     partly are not supported.
  *   - device_status, when not null, is a device int the kernel sets to 0. (The
  *     ranks no longer wait for one another, so there is no wait that could give
  *     up.)

@@ -1,0 +1,29 @@
+"""What the one-GPU calls decide on the host, before anything reaches a GPU."""
+import ctypes
+import os
+
+import pytest
+
+from dccl_b200.comm import FLOAT32, FLOAT64, OPS
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture
+def cuda_lib(dccl_lib):
+    if not hasattr(dccl_lib, "dccl_allreduce_one_device_noalloc"):
+        pytest.skip("library built without CUDA")
+    return dccl_lib
+
+
+@pytest.mark.parametrize("dtype,size", [(FLOAT32, 4), (FLOAT64, 8)])
+@pytest.mark.parametrize("where", ["input", "output"])
+def test_one_device_all_reduce_refuses_a_pointer_between_elements(cuda_lib, capfd, dtype, size, where):
+    fn = cuda_lib.dccl_allreduce_one_device_noalloc
+    fn.restype = ctypes.c_int
+    fn.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_size_t, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    good, odd = (ctypes.c_void_p * 2)(0x10000, 0x20000), (ctypes.c_void_p * 2)(0x10000, 0x20000 + size // 2)
+    ins, outs = (odd, good) if where == "input" else (good, odd)
+    assert fn(2, dtype, OPS["sum"], 4, ins, outs, None, None) == -1        # bad argument; the addresses are never used
+    assert "rank 1" in capfd.readouterr().err
+    assert fn(2, dtype, OPS["sum"], 0, ins, outs, None, None) == 0         # no element, nothing to refuse
