@@ -9,7 +9,9 @@ namespace dccl {
 
 /** First statement of such a kernel, before any access to memory, in every thread: the work before it in the stream is
  *  done and visible. (The kernels do not announce themselves early to the launch after them: whatever follows starts, as
- *  after any kernel, when they are done.) */
+ *  after any kernel, when they are done.) No pointer of such a kernel is __restrict__ and none is read by __ldg: either
+ *  declares its memory unchanged from the kernel's start on, which lies before that work, and lets a load be taken before
+ *  the wait. */
 __device__ __forceinline__ void wait_for_stream() { cudaGridDependencySynchronize(); }
 
 /**

@@ -63,7 +63,7 @@ static Cut cut_range(const void* dst, const void* src, size_t bytes) {
  * took 88.2 us.
  */
 constexpr int kCopyThreads = 256, kCopyU = 2;
-__global__ void __launch_bounds__(kCopyThreads) k_local_copy(char* __restrict__ dst, const char* __restrict__ src, const __grid_constant__ Cut c) {
+__global__ void __launch_bounds__(kCopyThreads) k_local_copy(char* dst, const char* src, const __grid_constant__ Cut c) {
     wait_for_stream();
     const size_t i0 = (size_t)blockIdx.x * (kCopyThreads * kCopyU) + threadIdx.x;
     uint4 v[kCopyU];

@@ -27,3 +27,20 @@ def test_one_device_all_reduce_refuses_a_pointer_between_elements(cuda_lib, capf
     assert fn(2, dtype, OPS["sum"], 4, ins, outs, None, None) == -1        # bad argument; the addresses are never used
     assert "rank 1" in capfd.readouterr().err
     assert fn(2, dtype, OPS["sum"], 0, ins, outs, None, None) == 0         # no element, nothing to refuse
+
+
+def test_early_launched_kernels_promise_nothing_about_their_inputs():
+    """A kernel that starts before the one ahead of it has written must not declare what it reads read-only for as long as it
+    runs: such loads may be taken before the wait."""
+    found = 0
+    folder = os.path.join(ROOT, "csrc", "kernels")
+    for name in sorted(os.listdir(folder)):
+        text = open(os.path.join(folder, name)).read()
+        for part in text.split("__global__")[1:]:
+            signature, body = part.split("{", 1)
+            body = body.split("\n}", 1)[0]
+            if "wait_for_stream()" not in body:
+                continue
+            found += 1
+            assert "__restrict__" not in signature + body and "__ldg" not in body, (name, signature)
+    assert found == 4
