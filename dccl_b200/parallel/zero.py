@@ -20,12 +20,26 @@ symmetric memory (``symmetric=True``), so that both collectives run zero-copy th
 import math
 
 import torch
+import torch.optim.adam as _adam
 import torch.optim.optimizer as _optimizer
 
 from .._lib import lib
 from ..comm import DcclError, current_stream_handle, dtype_of
 
 _FUSED_DTYPES = (torch.bfloat16, torch.float16, torch.float32)
+_IN_OPTIMIZER, _IN_ADAM = vars(_optimizer), vars(_adam)
+
+
+def _step_is_torchs_own():
+    """Whether AdamW's class still has the step that torch wrote, under nothing but the wrappers that torch's base class puts
+    around it: a function of another module in its place, or around it, has to run."""
+    try:
+        f = torch.optim.AdamW.step
+        while f.__globals__ is _IN_OPTIMIZER:
+            f = f.__wrapped__
+        return f.__globals__ is _IN_ADAM
+    except AttributeError:
+        return False
 
 
 class ShardedOptimizer:
@@ -99,7 +113,7 @@ class ShardedOptimizer:
         would have to see the gradient before or the result in between. None: the general path, which also reports
         whatever is wrong with the state."""
         inner = self.inner
-        if type(inner) is not torch.optim.AdamW or torch.compiler.is_compiling():
+        if type(inner) is not torch.optim.AdamW or not _step_is_torchs_own() or torch.compiler.is_compiling():
             return None
         if (inner._optimizer_step_pre_hooks or inner._optimizer_step_post_hooks or _optimizer._global_optimizer_pre_hooks
                 or _optimizer._global_optimizer_post_hooks):

@@ -1,5 +1,7 @@
 """The one-kernel AdamW update of dccl_b200.parallel.zero against the general path (torch's own optimizer and the casts
 around it), and which optimizers may take it."""
+import functools
+
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -148,3 +150,55 @@ def test_everything_else_stays_on_the_general_path(kw, cls):
     before = opt.groups[0]["flat"].clone()
     _train(opt, 2)
     assert opt._adamw_updates() is None and not torch.equal(before, opt.groups[0]["flat"])
+
+
+def _stepped(general, cls=torch.optim.AdamW, dtype=torch.float32, **kw):
+    """One step done: the state exists, and is the same bits on every path, because the first step is torch's own."""
+    return _train(_make(1, dtype, [1001], general, cls=cls, **kw), 1)
+
+
+def _same_after_a_step(a, b):
+    """One more step on both, and the same bits from it."""
+    before = a.groups[0]["flat"].clone()
+    for opt in (a, b):
+        _train(opt, 1)
+    for key in ("flat", "master"):
+        assert torch.equal(a.groups[0][key], b.groups[0][key])
+    assert not torch.equal(a.groups[0]["flat"], before)
+
+
+@pytest.fixture
+def cuda_lib(dccl_lib):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    assert _stepped(False)._adamw_updates() is not None        # what every case below changes one thing of
+
+
+def test_a_function_put_in_place_of_the_class_step_or_around_it_is_noticed(monkeypatch):
+    _make(1, torch.float32, [5], False, device="cpu")          # from the first object on, torch's base class wraps the step
+    assert zero._step_is_torchs_own()
+    stock = torch.optim.AdamW.step
+
+    def step(self, *args):
+        return stock(self, *args)
+
+    for other in (step, functools.wraps(stock)(step), functools.partialmethod(stock), torch.optim.Optimizer.profile_hook_step(step)):
+        monkeypatch.setattr(torch.optim.AdamW, "step", other)
+        assert not zero._step_is_torchs_own()
+    monkeypatch.setattr(torch.optim.AdamW, "step", stock)
+    assert zero._step_is_torchs_own()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("wraps", [False, True])
+def test_a_step_replaced_on_the_class_runs(cuda_lib, monkeypatch, wraps):
+    a, b = _stepped(False), _stepped(True)
+    stock, calls = torch.optim.AdamW.step, []
+
+    def step(self, *args):
+        calls.append(self)
+        return stock(self, *args)
+
+    monkeypatch.setattr(torch.optim.AdamW, "step", functools.wraps(stock)(step) if wraps else step)
+    _same_after_a_step(a, b)
+    assert calls == [a.inner, b.inner]
