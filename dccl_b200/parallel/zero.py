@@ -22,6 +22,7 @@ import math
 import torch
 import torch.optim.adam as _adam
 import torch.optim.optimizer as _optimizer
+from torch.utils._device import DeviceContext
 
 from .._lib import lib
 from ..comm import DcclError, current_stream_handle, dtype_of
@@ -40,6 +41,15 @@ def _step_is_torchs_own():
         return f.__globals__ is _IN_ADAM
     except AttributeError:
         return False
+
+
+def _a_mode_is_active():
+    """Whether a mode would see torch's calls: any, except the one behind ``torch.device`` and the default device, which only
+    places new tensors."""
+    if torch._C._len_torch_dispatch_stack():
+        return True
+    n = torch._C._len_torch_function_stack()
+    return n > 0 and any(type(torch._C._get_function_stack_at(i)) is not DeviceContext for i in range(n))
 
 
 class ShardedOptimizer:
@@ -114,6 +124,8 @@ class ShardedOptimizer:
         whatever is wrong with the state."""
         inner = self.inner
         if type(inner) is not torch.optim.AdamW or not _step_is_torchs_own() or torch.compiler.is_compiling():
+            return None
+        if _a_mode_is_active():
             return None
         if (inner._optimizer_step_pre_hooks or inner._optimizer_step_post_hooks or _optimizer._global_optimizer_pre_hooks
                 or _optimizer._global_optimizer_post_hooks):

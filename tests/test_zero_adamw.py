@@ -6,6 +6,9 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
+from torch.overrides import TorchFunctionMode  # noqa: E402
+from torch.utils._python_dispatch import TorchDispatchMode  # noqa: E402
+
 from dccl_b200.parallel import zero  # noqa: E402
 
 
@@ -202,3 +205,49 @@ def test_a_step_replaced_on_the_class_runs(cuda_lib, monkeypatch, wraps):
     monkeypatch.setattr(torch.optim.AdamW, "step", functools.wraps(stock)(step) if wraps else step)
     _same_after_a_step(a, b)
     assert calls == [a.inner, b.inner]
+
+
+class SeesDispatch(TorchDispatchMode):
+    """Counts what passes it."""
+    seen = 0
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.seen += 1
+        return func(*args, **(kwargs or {}))
+
+
+class SeesFunctions(TorchFunctionMode):
+    seen = 0
+
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        self.seen += 1
+        return func(*args, **(kwargs or {}))
+
+
+def test_which_modes_count():
+    assert not zero._a_mode_is_active()
+    for mode in (SeesDispatch, SeesFunctions):
+        with mode():
+            assert zero._a_mode_is_active()
+            with torch.device("cpu"):
+                assert zero._a_mode_is_active()
+        with torch.device("cpu"):
+            assert not zero._a_mode_is_active()
+            with mode():
+                assert zero._a_mode_is_active()
+    assert not zero._a_mode_is_active()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [SeesDispatch, SeesFunctions])
+def test_an_active_mode_sees_the_operations_of_the_step(cuda_lib, mode):
+    a, b = _stepped(False), _stepped(True)
+    with mode() as m:
+        a.step()
+    assert m.seen > 3
+    b.step()
+    assert torch.equal(a.groups[0]["flat"], b.groups[0]["flat"])
+    with torch.device("cuda"):                                  # a mode, too, but one that only places new tensors
+        assert a._adamw_updates() is not None
+        with mode():
+            assert a._adamw_updates() is None
