@@ -29,6 +29,7 @@ from ..comm import DcclError, current_stream_handle, dtype_of
 
 _FUSED_DTYPES = (torch.bfloat16, torch.float16, torch.float32)
 _IN_OPTIMIZER, _IN_ADAM = vars(_optimizer), vars(_adam)
+_enter_range, _exit_range = torch._C._autograd._record_function_with_args_enter, torch._C._autograd._record_function_with_args_exit
 
 
 def _step_is_torchs_own():
@@ -105,8 +106,7 @@ class ShardedOptimizer:
                 comm.reduce_scatter(g["grad"], g["grad_slice"], op="avg")
         updates = self._adamw_updates()
         if updates is not None:
-            for u in updates:
-                self._adamw(*u)
+            self._adamw_range(updates)
         else:
             for g in self.groups:
                 g["master"].grad.copy_(g["grad_slice"] if n > 1 else g["grad"])
@@ -159,6 +159,19 @@ class ShardedOptimizer:
         if step is not None:
             inner._opt_called = True
         return updates
+
+    def _adamw_range(self, updates):
+        """The updates, where torch's optimizers show their step: inside the range that the profiler and other observers know
+        it by, with the call at its end through which the profiler finds the optimizer. The range is there whether or not
+        anything looks, because an observer may without being the profiler. Entered this way it costs a step 1.4 us;
+        torch's record_function enters the same one in 5 us."""
+        entered = _enter_range("Optimizer.step#AdamW.step")
+        try:
+            for u in updates:
+                self._adamw(*u)
+            self.inner._optimizer_step_code()
+        finally:
+            _exit_range(entered)
 
     def _adamw(self, g, o, st):
         p, n = g["master"], self.comm.world

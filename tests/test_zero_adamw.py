@@ -251,3 +251,26 @@ def test_an_active_mode_sees_the_operations_of_the_step(cuda_lib, mode):
         assert a._adamw_updates() is not None
         with mode():
             assert a._adamw_updates() is None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("observer", ["profiler", "execution trace"])
+def test_the_profiler_range_of_the_step_is_there_on_both_paths(cuda_lib, monkeypatch, tmp_path, observer):
+    for general in (False, True):
+        opt, told = _stepped(general), []
+        monkeypatch.setattr(opt.inner, "_optimizer_step_code", lambda: told.append(1), raising=False)
+        if observer == "profiler":
+            with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+                opt.step()
+            ranges = [e for e in prof.events() if e.name == "Optimizer.step#AdamW.step"]
+            assert len(ranges) == 1 and ranges[0].is_user_annotation
+        else:
+            path = str(tmp_path / ("%s.json" % general))
+            trace = torch.profiler.ExecutionTraceObserver()
+            trace.register_callback(path)
+            trace.start()
+            opt.step()
+            trace.stop()
+            trace.unregister_callback()
+            assert "Optimizer.step#AdamW.step" in open(path).read()
+        assert told == [1]
