@@ -189,6 +189,14 @@ int fail(const char* what) {
     return -1;
 }
 
+/** A launch can be refused before the runtime is asked, so the reason comes from the call and not from the last error. */
+int fail_reduce(cudaError_t e, const void* acc, const void* in, size_t es) {
+    if (es && (reinterpret_cast<uintptr_t>(acc) | reinterpret_cast<uintptr_t>(in)) % es) fprintf(stderr, "dccl local reduce: a buffer lies between two elements of %zu bytes\n", es);
+    else fprintf(stderr, "dccl local reduce: %s\n", cudaGetErrorString(e));
+    cudaGetLastError();
+    return -1;
+}
+
 } // namespace
 
 extern "C" {
@@ -639,12 +647,13 @@ int dccl_local_reduce(void* host_acc, const void* host_in, size_t count, int dty
     if (e == cudaSuccess) cudaMemcpy(host_acc, a, count * es, cudaMemcpyDeviceToHost);
     cudaFree(a);
     cudaFree(b);
-    return e == cudaSuccess ? 0 : fail("local reduce");
+    return e == cudaSuccess ? 0 : fail_reduce(e, a, b, es);
 }
 
 /** The same kernel on buffers that already live on the device, on `stream` (no synchronisation): for timing. */
 int dccl_local_reduce_device(void* dev_acc, const void* dev_in, size_t count, int dtype, int op, void* stream) {
-    return launch_local_reduce(dev_acc, dev_in, count, (ncclDataType_t)dtype, (ncclRedOp_t)op, (cudaStream_t)stream) == cudaSuccess ? 0 : fail("local reduce");
+    const cudaError_t e = launch_local_reduce(dev_acc, dev_in, count, (ncclDataType_t)dtype, (ncclRedOp_t)op, (cudaStream_t)stream);
+    return e == cudaSuccess ? 0 : fail_reduce(e, dev_acc, dev_in, size_of_type((ncclDataType_t)dtype));
 }
 
 } // extern "C"

@@ -44,3 +44,8 @@ def test_early_launched_kernels_promise_nothing_about_their_inputs():
             found += 1
             assert "__restrict__" not in signature + body and "__ldg" not in body, (name, signature)
     assert found == 4
+
+
+def test_pairwise_fold_says_why_it_refuses_a_pointer(cuda_lib, capfd):
+    assert cuda_lib.dccl_local_reduce_device(0x10002, 0x20000, 8, FLOAT32, OPS["sum"], None) != 0
+    assert "between two elements of 4 bytes" in capfd.readouterr().err
