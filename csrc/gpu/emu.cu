@@ -647,7 +647,7 @@ int dccl_local_reduce(void* host_acc, const void* host_in, size_t count, int dty
     if (e == cudaSuccess) cudaMemcpy(host_acc, a, count * es, cudaMemcpyDeviceToHost);
     cudaFree(a);
     cudaFree(b);
-    return e == cudaSuccess ? 0 : fail_reduce(e, a, b, es);
+    return e == cudaSuccess ? 0 : fail_reduce(e, nullptr, nullptr, es);      // allocations are aligned
 }
 
 /** The same kernel on buffers that already live on the device, on `stream` (no synchronisation): for timing. */
