@@ -55,7 +55,8 @@ extern "C" {
 
 #define DCCL_NOALLOC_MAX_RANKS 8
 #define DCCL_NOALLOC_MAX_BYTES (256u * 1024u)
-/* device memory the library holds for this entry point: none */
+/* device memory the library holds for this entry point, for one rank and altogether: none */
+#define DCCL_NOALLOC_RANK_BYTES 0u
 #define DCCL_NOALLOC_SCRATCH_BYTES 0u
 
 #define DCCL_NOALLOC_OK 0

@@ -1,6 +1,7 @@
 """What the one-GPU calls decide on the host, before anything reaches a GPU."""
 import ctypes
 import os
+import subprocess
 
 import pytest
 
@@ -49,3 +50,13 @@ def test_early_launched_kernels_promise_nothing_about_their_inputs():
 def test_pairwise_fold_says_why_it_refuses_a_pointer(cuda_lib, capfd):
     assert cuda_lib.dccl_local_reduce_device(0x10002, 0x20000, 8, FLOAT32, OPS["sum"], None) != 0
     assert "between two elements of 4 bytes" in capfd.readouterr().err
+
+
+def test_one_device_header_keeps_its_names(tmp_path):
+    """As C, with every name that a caller may have sized something by."""
+    src = tmp_path / "names.c"
+    src.write_text("""#include "noalloc_allreduce.h"
+unsigned sizes[] = {DCCL_NOALLOC_MAX_RANKS, DCCL_NOALLOC_MAX_BYTES, DCCL_NOALLOC_RANK_BYTES, DCCL_NOALLOC_SCRATCH_BYTES};
+int codes[] = {DCCL_NOALLOC_OK, DCCL_NOALLOC_BAD_ARGUMENT, DCCL_NOALLOC_TOO_LARGE, DCCL_NOALLOC_CUDA_ERROR};
+""")
+    subprocess.run(["gcc", "-Wall", "-Werror", "-c", "-I", os.path.join(ROOT, "csrc", "kernels"), "-o", str(tmp_path / "names.o"), str(src)], check=True)
