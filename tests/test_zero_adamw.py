@@ -1,11 +1,13 @@
 """The one-kernel AdamW update of dccl_b200.parallel.zero against the general path (torch's own optimizer and the casts
 around it), and which optimizers may take it."""
 import functools
+import warnings
 
 import pytest
 
 torch = pytest.importorskip("torch")
 
+from torch.optim.optimizer import register_optimizer_step_post_hook, register_optimizer_step_pre_hook  # noqa: E402
 from torch.overrides import TorchFunctionMode  # noqa: E402
 from torch.utils._python_dispatch import TorchDispatchMode  # noqa: E402
 
@@ -143,7 +145,7 @@ def test_two_slices_changed_options_and_loaded_state(dccl_lib):
 @pytest.mark.parametrize("kw,cls", [({"amsgrad": True}, torch.optim.AdamW), ({"maximize": True}, torch.optim.AdamW), ({}, torch.optim.Adam),
                                     ({"lr": torch.tensor(1e-2)}, torch.optim.AdamW), ({}, torch.optim.SGD), ({}, torch.optim.AdamW)])
 def test_everything_else_stays_on_the_general_path(kw, cls):
-    """Options the kernel does not implement, other optimizers, and host tensors."""
+    """Host tensors, with any options and optimizer. (What keeps tensors on a GPU from the kernel: further below.)"""
     opts = dict(kw)
     if cls is torch.optim.SGD:
         params = [torch.nn.Parameter(torch.randn(5))]
@@ -274,3 +276,130 @@ def test_the_profiler_range_of_the_step_is_there_on_both_paths(cuda_lib, monkeyp
             trace.unregister_callback()
             assert "Optimizer.step#AdamW.step" in open(path).read()
         assert told == [1]
+
+
+def _option(name, value):
+    def change(opt, monkeypatch):
+        opt.inner.param_groups[0][name] = value() if callable(value) else value
+    return change
+
+
+def _state(name, value):
+    def change(opt, monkeypatch):
+        st = opt.inner.state[opt.groups[0]["master"]]
+        st[name] = value(st[name])
+    return change
+
+
+def _replaced_on_the_instance(opt, monkeypatch):
+    opt.inner.step = functools.partial(type(opt.inner).step, opt.inner)
+
+
+def _another_group(opt, monkeypatch):
+    opt.inner.add_param_group({"params": [torch.nn.Parameter(torch.zeros(3, device="cuda"))]})
+
+
+def _another_parameter(opt, monkeypatch):
+    opt.inner.param_groups[0]["params"].append(torch.nn.Parameter(torch.zeros(3, device="cuda")))
+
+
+def _hook(register):
+    def change(opt, monkeypatch):
+        monkeypatch.callbacks.append(register(opt.inner)(lambda *a: None))
+    return change
+
+
+def _between(x):
+    return torch.stack([x, x], 1)[:, 0]                         # every second element of twice as many
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("change", [
+    _option("maximize", True), _option("decoupled_weight_decay", False), _option("lr", lambda: torch.tensor(1e-2)), _another_group, _another_parameter, _replaced_on_the_instance,
+    _hook(lambda o: o.register_step_pre_hook), _hook(lambda o: o.register_step_post_hook),
+    _hook(lambda o: register_optimizer_step_pre_hook), _hook(lambda o: register_optimizer_step_post_hook),
+    _state("exp_avg", _between), _state("exp_avg_sq", _between),
+], ids=["maximize", "coupled decay", "tensor lr", "two groups", "two parameters", "replaced step", "pre hook", "post hook", "global pre hook", "global post hook", "strided m", "strided v"])
+def test_one_change_takes_the_general_path(cuda_lib, monkeypatch, change):
+    monkeypatch.callbacks = []
+    a, b = _stepped(False), _stepped(True)
+    try:
+        for opt in (a, b):
+            change(opt, monkeypatch)
+        assert a._adamw_updates() is None
+        _same_after_a_step(a, b)
+    finally:
+        for c in monkeypatch.callbacks:
+            c.remove()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("change", [
+    # torch refuses some of these; the kernel must not get them before it does
+    _option("amsgrad", True), _option("capturable", True), _option("differentiable", True), _option("fused", True), _option("weight_decay", lambda: torch.tensor(0.1)),
+    _option("eps", lambda: torch.tensor(1e-8)), _option("betas", lambda: (torch.tensor(0.9), 0.95)), _option("betas", lambda: (0.9, torch.tensor(0.95))),
+    _state("step", lambda x: x.cuda()), _state("step", float), _state("exp_avg", lambda x: x[:-1]), _state("exp_avg", lambda x: x.double()),
+    _state("exp_avg", lambda x: None), _state("exp_avg_sq", lambda x: x.cpu()), _state("exp_avg_sq", lambda x: torch.nn.Parameter(x)),
+], ids=["amsgrad", "capturable", "differentiable", "fused", "tensor decay", "tensor eps", "tensor beta 1", "tensor beta 2", "step on the GPU", "step a number", "m too short",
+        "m in fp64", "no m", "v on the host", "v of a subclass"])
+def test_options_and_state_the_kernel_does_not_take(cuda_lib, monkeypatch, change):
+    opt = _stepped(False)
+    change(opt, monkeypatch)
+    assert opt._adamw_updates() is None
+
+
+@pytest.mark.gpu
+def test_optimizers_dtypes_and_surroundings_the_kernel_does_not_take(cuda_lib, monkeypatch):
+    assert _stepped(False, cls=torch.optim.Adam)._adamw_updates() is None
+    assert _stepped(False, cls=type("Derived", (torch.optim.AdamW,), {}))._adamw_updates() is None
+    assert _stepped(False, dtype=torch.float64)._adamw_updates() is None
+    assert _make(1, torch.float32, [5], False)._adamw_updates() is None            # no state yet
+    opt = _stepped(False)
+    opt.groups[0]["master"].grad = None
+    assert opt._adamw_updates() is None
+    opt = _stepped(False)
+    other = opt.groups[0]["master"].detach().clone().requires_grad_(True)
+    other.grad = torch.zeros_like(other)
+    opt.inner.state[other] = opt.inner.state[opt.groups[0]["master"]]
+    opt.inner.param_groups[0]["params"][0] = other
+    assert opt._adamw_updates() is None
+    opt = _stepped(False)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = opt._adamw_updates()
+        torch.zeros(1, device="cuda")
+    assert captured is None and opt._adamw_updates() is not None
+    monkeypatch.setattr(torch.compiler, "is_compiling", lambda: True)
+    assert opt._adamw_updates() is None
+
+
+@pytest.mark.gpu
+def test_the_update_is_ordered_on_a_side_stream(cuda_lib):
+    a, b = _stepped(False), _stepped(True)
+    grad = torch.randn(a.groups[0]["grad"].numel(), device="cuda")
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        for _ in range(3):
+            torch.cuda._sleep(2000000)                          # about a millisecond: a launch elsewhere would come first
+            a.groups[0]["grad"].copy_(grad)
+            a.step()
+            a.groups[0]["grad"].fill_(float("nan"))
+    side.synchronize()
+    for _ in range(3):
+        b.groups[0]["grad"].copy_(grad)
+        b.step()
+    torch.testing.assert_close(a.groups[0]["flat"], b.groups[0]["flat"], rtol=4 * 2.0 ** -23, atol=1e-7)
+
+
+@pytest.mark.gpu
+def test_a_scheduler_made_late_sees_the_next_step(cuda_lib):
+    """Its first step warns unless the optimizer has stepped since it was made, on either path."""
+    for general in (False, True):
+        opt = _stepped(general)
+        sched = torch.optim.lr_scheduler.LambdaLR(opt.inner, lambda t: 0.5 ** t)
+        with warnings.catch_warnings():
+            warnings.simplefilter("error")
+            _train(opt, 1)
+            sched.step()
+        assert opt.inner.param_groups[0]["lr"] == 0.5e-2
