@@ -83,8 +83,7 @@ def test_two_calls_in_a_row_match_the_allocating_entry_point(dccl_lib):
     if not torch.cuda.is_available():
         pytest.skip("needs a GPU")
     torch.cuda.set_device(0)
-    # first call (this is also the per-device set-up), then a second one that reuses the same array with
-    # another shape, so stale flags or staging bytes from the first call would show
+    # two calls of different shapes, so that anything left over from the first would show
     _run(dccl_lib, torch, 8, "float32", "sum", MAX_BYTES // 4, seed=1)
     _run(dccl_lib, torch, 3, "bfloat16", "avg", 10007, seed=2)
     # and more pairs: every width, in place, one rank, tiny messages
@@ -93,10 +92,10 @@ def test_two_calls_in_a_row_match_the_allocating_entry_point(dccl_lib):
     _run(dccl_lib, torch, 2, "float64", "prod", 1000, seed=5)
     _run(dccl_lib, torch, 1, "float16", "sum", 5, seed=6)
     _run(dccl_lib, torch, 5, "uint8", "min", 3, seed=7)
-    _run(dccl_lib, torch, 2, "float32", "sum", MAX_BYTES // 4, seed=8)   # the limit, worst case for staging
+    _run(dccl_lib, torch, 2, "float32", "sum", MAX_BYTES // 4, seed=8)   # the limit with the fewest ranks
 
 
-def test_requests_beyond_the_built_in_scratch_are_refused(dccl_lib, capfd):
+def test_requests_beyond_the_limits_are_refused(dccl_lib, capfd):
     torch = pytest.importorskip("torch")
     if not torch.cuda.is_available():
         pytest.skip("needs a GPU")
@@ -105,7 +104,7 @@ def test_requests_beyond_the_built_in_scratch_are_refused(dccl_lib, capfd):
     ptrs = (ctypes.c_void_p * 2)(t.data_ptr(), t.data_ptr())
     assert fn(2, 7, 0, MAX_BYTES // 4 + 1, ptrs, ptrs, None, None) == -2     # too large: nothing is launched
     assert "above the limit" in capfd.readouterr().err
-    assert fn(9, 7, 0, 4, ptrs, ptrs, None, None) == -1                        # more ranks than the array holds
+    assert fn(9, 7, 0, 4, ptrs, ptrs, None, None) == -1                        # more ranks than the limit
     assert fn(2, 7, 0, 0, ptrs, ptrs, None, None) == 0                         # nothing to do
     torch.cuda.synchronize()
 
@@ -194,3 +193,50 @@ def test_one_rank_copies_from_and_to_any_address(dccl_lib, name, count, in_off, 
     rc = _entry(dccl_lib)(1, DTYPE_NAMES.index(name), OPS["sum"], count, (ctypes.c_void_p * 1)(src.data_ptr() + in_off),
                           (ctypes.c_void_p * 1)(dst.data_ptr() + out_off), None, torch.cuda.current_stream().cuda_stream)
     assert rc == 0 and torch.equal(dst, want)
+
+
+def _call(lib, torch, ins, outs, stream):
+    n = len(ins)
+    rc = _entry(lib)(n, DTYPE_NAMES.index("float32"), OPS["sum"], ins[0].numel(), (ctypes.c_void_p * n)(*[t.data_ptr() for t in ins]),
+                     (ctypes.c_void_p * n)(*[t.data_ptr() for t in outs]), None, stream.cuda_stream)
+    assert rc == 0
+
+
+def test_calls_on_different_streams_overlap(dccl_lib):
+    """Three streams, each with chains of its own calls and nothing that orders them: calls share no state."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    # whole numbers, which are exact: in place, every call after a chain's first multiplies by the number of ranks
+    bufs = [[torch.full((MAX_BYTES // 4 - s,), float(10 * s + r), device="cuda") for r in range(4)] for s in range(3)]
+    torch.cuda.synchronize()
+    for s in streams:
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(1000000)              # all chains are queued before the first runs
+    for k in range(4):
+        for s, b in zip(streams, bufs):
+            _call(dccl_lib, torch, b, b, s)
+    torch.cuda.synchronize()
+    for s, b in enumerate(bufs):
+        for t in b:
+            assert torch.all(t == 64.0 * (40 * s + 6))
+
+
+def test_calls_are_captured_in_a_graph(dccl_lib):
+    """Two that depend on each other, replayed on new values."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    ins = [torch.zeros(10007, device="cuda") for _ in range(5)]
+    outs = [torch.empty_like(t) for t in ins]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        _call(dccl_lib, torch, ins, outs, torch.cuda.current_stream())
+        _call(dccl_lib, torch, outs, ins, torch.cuda.current_stream())
+    for k in range(1, 4):
+        for r, t in enumerate(ins):
+            t.fill_(float(k * r))
+        graph.replay()
+        for o, i in zip(outs, ins):
+            assert torch.all(o == 10.0 * k) and torch.all(i == 50.0 * k)
