@@ -108,6 +108,8 @@ def _declare(lib):
         "dccl_local_reduce": (i, [vp, vp, sz, i, i]),
         "dccl_local_reduce_device": (i, [vp, vp, sz, i, i, vp]),
         "dccl_adamw_flat": (i, [i, i, sz, vp, vp, vp, vp, vp, vp] + [c.c_double] * 7 + [vp]),
+        "dccl_emu_early_producer": (i, [vp, vp, sz, c.c_uint, vp, vp]),
+        "dccl_emu_early_observer": (i, [vp, vp]),
         "dccl_debug_bounds_build": (i, []),
         "dccl_selftest_canary": (i, []),
         "dccl_emu_set_guard": (None, [i]),
