@@ -54,9 +54,6 @@ template <typename A> __device__ __forceinline__ A avg_finish(A a, int n) {
     else return (A)(a / (A)n);
 }
 
-/** N elements moved by one access. */
-template <typename T, int N> struct alignas(sizeof(T) * N) Pack { T e[N]; };
-
 template <typename T> struct alignas(16) Vec16 {
     static constexpr int N = 16 / (int)sizeof(T);
     T e[N];

@@ -23,6 +23,9 @@ struct AdamWArgs {
     float eps;
 };
 
+/** N elements moved by one access. */
+template <typename T, int N> struct alignas(sizeof(T) * N) Pack { T e[N]; };
+
 constexpr int kAdamWThreads = 128;
 constexpr int kAdamWN = 4;              // elements of one access: 16 bytes of fp32
 
@@ -94,11 +97,9 @@ extern "C" int dccl_adamw_flat(int device, int dtype, size_t n, void* master, vo
                    (float)decay, (float)w1, (float)b2, (float)w2, (float)step, (float)bc2_sqrt, (float)eps};
     const uintptr_t low = (uintptr_t)master | (uintptr_t)master_grad | (uintptr_t)m | (uintptr_t)v;
     const uintptr_t half = (uintptr_t)grad | (uintptr_t)out;
-    bool vec = low % 16 == 0 && half % (dtype == 7 ? 16 : 8) == 0;
+    const bool vec = low % 16 == 0 && half % (dtype == 7 ? 16 : 8) == 0;
     const size_t per = (size_t)kAdamWThreads * kAdamWN;
-    const size_t blocks = (n + per - 1) / per;
-    const unsigned grid = (unsigned)(blocks < 0x7fffffffu ? blocks : 0x7fffffffu);
-    if (grid < blocks) vec = false;
+    const unsigned grid = (unsigned)((n + per - 1) / per);      // enough for 10^12 elements
     int prev = -1;
     cudaGetDevice(&prev);
     cudaError_t e = prev != device ? cudaSetDevice(device) : cudaSuccess;

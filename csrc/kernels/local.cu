@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(kCopyThreads) k_local_copy(char* dst, const ch
 #pragma unroll
     for (int u = 0; u < kCopyU; u++)
         if (i0 + u * kCopyThreads < c.nv) *reinterpret_cast<uint4*>(dst + c.head + (i0 + u * kCopyThreads) * 16) = v[u];
-    if (blockIdx.x == 0) {      // at most 31 bytes before and 47 behind the vectors
+    if (blockIdx.x == 0) {      // at most 30 bytes before and 30 behind the vectors
         for (size_t j = threadIdx.x; j < c.head; j += kCopyThreads) dst[j] = src[j];
         for (size_t j = c.head + c.nv * 16 + threadIdx.x; j < c.head + c.nv * 16 + c.rest; j += kCopyThreads) dst[j] = src[j];
     }
