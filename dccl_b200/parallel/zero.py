@@ -17,7 +17,9 @@ tensors the device kernels on the current stream; on GPUs with NVSwitch multicas
 symmetric memory (``symmetric=True``), so that both collectives run zero-copy through the switch. Call
 ``close()`` before the communicator is finalized to give that memory back.
 """
+import ctypes
 import math
+import os
 
 import torch
 import torch.optim.adam as _adam
@@ -30,6 +32,20 @@ from ..comm import DcclError, current_stream_handle, dtype_of
 _FUSED_DTYPES = (torch.bfloat16, torch.float16, torch.float32)
 _IN_OPTIMIZER, _IN_ADAM = vars(_optimizer), vars(_adam)
 _enter_range, _exit_range = torch._C._autograd._record_function_with_args_enter, torch._C._autograd._record_function_with_args_exit
+
+
+def _observer_query():
+    """hasCallbacks of torch's C++ API (ATen/record_function.h): whether anything looks at ranges, be it the profiler or an
+    observer without it. A torch that does not export it is taken to be observed always."""
+    try:
+        f = ctypes.PyDLL(os.path.join(os.path.dirname(torch.__file__), "lib", "libtorch_cpu.so"))._ZN2at12hasCallbacksEv
+    except (OSError, AttributeError):
+        return lambda: True
+    f.restype, f.argtypes = ctypes.c_bool, []
+    return f
+
+
+_observed = _observer_query()
 
 
 def _step_is_torchs_own():
@@ -162,16 +178,16 @@ class ShardedOptimizer:
 
     def _adamw_range(self, updates):
         """The updates, where torch's optimizers show their step: inside the range that the profiler and other observers know
-        it by, with the call at its end through which the profiler finds the optimizer. The range is there whether or not
-        anything looks, because an observer may without being the profiler. Entered this way it costs a step 2.4 us;
-        torch's record_function enters the same one in 5 us."""
-        entered = _enter_range("Optimizer.step#AdamW.step")
+        it by, with the call at its end through which the profiler finds the optimizer. An unobserved range costs a step
+        2.4 us of 15.8 and is left out."""
+        entered = _enter_range("Optimizer.step#AdamW.step") if _observed() else None
         try:
             for u in updates:
                 self._adamw(*u)
             self.inner._optimizer_step_code()
         finally:
-            _exit_range(entered)
+            if entered is not None:
+                _exit_range(entered)
 
     def _adamw(self, g, o, st):
         p, n = g["master"], self.comm.world

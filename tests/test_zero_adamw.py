@@ -255,6 +255,19 @@ def test_an_active_mode_sees_the_operations_of_the_step(cuda_lib, mode):
             assert a._adamw_updates() is None
 
 
+def test_ranges_are_entered_while_something_observes_them(tmp_path):
+    assert not zero._observed()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]):
+        assert zero._observed()
+    trace = torch.profiler.ExecutionTraceObserver()
+    trace.register_callback(str(tmp_path / "trace.json"))
+    trace.start()
+    seen = zero._observed()
+    trace.stop()
+    trace.unregister_callback()
+    assert seen and not zero._observed()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("observer", ["profiler", "execution trace"])
 def test_the_profiler_range_of_the_step_is_there_on_both_paths(cuda_lib, monkeypatch, tmp_path, observer):
