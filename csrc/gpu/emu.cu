@@ -650,7 +650,7 @@ int dccl_local_reduce(void* host_acc, const void* host_in, size_t count, int dty
     return e == cudaSuccess ? 0 : fail_reduce(e, nullptr, nullptr, es);      // allocations are aligned
 }
 
-/** The same kernel on buffers that already live on the device, on `stream` (no synchronisation): for timing. */
+/** The same kernel on buffers that already live on the device, on `stream` (no synchronisation): for tests and measurements. */
 int dccl_local_reduce_device(void* dev_acc, const void* dev_in, size_t count, int dtype, int op, void* stream) {
     const cudaError_t e = launch_local_reduce(dev_acc, dev_in, count, (ncclDataType_t)dtype, (ncclRedOp_t)op, (cudaStream_t)stream);
     return e == cudaSuccess ? 0 : fail_reduce(e, dev_acc, dev_in, size_of_type((ncclDataType_t)dtype));
