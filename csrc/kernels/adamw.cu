@@ -22,6 +22,7 @@ struct AdamWArgs {
     float bc2_sqrt;     // sqrt(1 - beta2^t)
     float eps;
 };
+static_assert(launch_is_cheap(sizeof(AdamWArgs) + sizeof(bool)), "parameters of k_adamw");
 
 /** N elements moved by one access. */
 template <typename T, int N> struct alignas(sizeof(T) * N) Pack { T e[N]; };

@@ -15,6 +15,13 @@ namespace dccl {
 __device__ __forceinline__ void wait_for_stream() { cudaGridDependencySynchronize(); }
 
 /**
+ * What a launch costs the host depends on the size of the kernel's parameters, with a period of 64 bytes: 17 to 32 bytes past a
+ * multiple of 64 took 1.54 us, every other size 1.81 to 1.94 us (8 to 320 bytes in steps of 8, calls back to back). A kernel
+ * whose calls are short packs its parameters into such a size.
+ */
+constexpr bool launch_is_cheap(size_t parameter_bytes) { return parameter_bytes % 64 > 16 && parameter_bytes % 64 <= 32; }
+
+/**
  * Measured on back-to-back calls: the pairwise fold of 25 MiB of bf16 14.35 -> 12.7 us, of 12 MB of unaligned fp16
  * 6.15 -> 4.4 us, the copy of 26 MB 12.3 -> 10.0 us; nothing at 1 GiB. A capturing stream gets an ordinary launch: the
  * edge a programmatic one leaves in a graph carries data that not every user of the capture API expects.
