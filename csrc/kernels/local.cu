@@ -85,38 +85,48 @@ __global__ void __launch_bounds__(kCopyThreads) k_local_copy(char* dst, const ch
 }
 
 /**
- * acc[i] = op(acc[i], in[i]): three streams of HBM traffic and nothing else. One vector of each operand per thread, the
- * CTAs following each other through memory as in the copy: 1 GiB fp32 takes 448 us (7.2 TB/s), 25 MiB bf16 12.7 us and
- * 1 MiB 3.6 us (the host's cost of the call), where two resident CTAs per SM with eight vectors in flight per thread, each
- * CTA on a piece of at least 64 KB, took 520, 16.4 and 5.1 us. Operands at different distances from a 16-byte boundary
- * read `in` through a window as the copy does: 12 MB of fp16 24.6 -> 4.4 us (before: one element per access). The elements
- * outside the vectors get threads of their own behind the vectors' threads.
+ * acc[i] = op(acc[i], in[i]): three streams of HBM traffic and nothing else, the CTAs following each other through memory as in
+ * the copy: 1 GiB fp32 takes 446 us (7.2 TB/s), 25 MiB bf16 12.7 us and 1 MiB 3.3 us (the host's cost of the call), where two
+ * resident CTAs per SM with eight vectors in flight per thread, each CTA on a piece of at least 64 KB, took 520, 16.4 and 5.1 us.
+ * Operands at different distances from a 16-byte boundary read `in` through a window as the copy does: 12 MB of fp16 24.6 ->
+ * 4.3 us (before: one element per access). The elements outside the vectors get threads of their own behind the vectors' threads.
  */
-constexpr int kReduceThreads = 512;
-template <typename T, int OP>
-__global__ void __launch_bounds__(kReduceThreads) k_local_reduce(T* acc, const T* in, const __grid_constant__ Cut c) {
+template <typename T, int OP, int THREADS, int U>
+__global__ void __launch_bounds__(THREADS) k_local_reduce(T* acc, const T* in, const __grid_constant__ Cut c) {
     using A = typename Traits<T>::Acc;
     constexpr int N = Vec16<T>::N;
     wait_for_stream();
-    const size_t t = (size_t)blockIdx.x * kReduceThreads + threadIdx.x;
+    const size_t t0 = (size_t)blockIdx.x * (THREADS * U) + threadIdx.x;
     const size_t head = c.head / sizeof(T);
-    if (t < c.nv) {
-        T* p = acc + head + t * N;
-        Window w;
-        load(w, reinterpret_cast<const char*>(in + head + t * N) - c.shift, c.shift);
-        Vec16<T> x = ld_vec<T>(p), y;
-        *reinterpret_cast<uint4*>(&y) = cut_out(w, c.shift);
-        if constexpr (kFoldsBytes<T, OP>) fold_bytes<T, OP>(x, y);
-        else {
+    T* p = acc + head;
+    const char* q = reinterpret_cast<const char*>(in + head) - c.shift;
+    Window w[U];
+    Vec16<T> x[U];
 #pragma unroll
-            for (int e = 0; e < N; e++) x.e[e] = Traits<T>::down(op_apply<OP, A>(Traits<T>::up(x.e[e]), Traits<T>::up(y.e[e])));
-        }
-        st_vec<T>(p, x);
-        return;
+    for (int u = 0; u < U; u++) {
+        const size_t t = t0 + u * THREADS;
+        if (t >= c.nv) continue;
+        load(w[u], q + t * 16, c.shift);
+        x[u] = ld_vec<T>(p + t * N);
     }
-    size_t i = t - c.nv;
-    if (i >= head) i += c.nv * N;
-    if (i < head + c.nv * N + c.rest / sizeof(T)) acc[i] = Traits<T>::down(op_apply<OP, A>(Traits<T>::up(acc[i]), Traits<T>::up(in[i])));
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const size_t t = t0 + u * THREADS;
+        if (t < c.nv) {
+            Vec16<T> y;
+            *reinterpret_cast<uint4*>(&y) = cut_out(w[u], c.shift);
+            if constexpr (kFoldsBytes<T, OP>) fold_bytes<T, OP>(x[u], y);
+            else {
+#pragma unroll
+                for (int e = 0; e < N; e++) x[u].e[e] = Traits<T>::down(op_apply<OP, A>(Traits<T>::up(x[u].e[e]), Traits<T>::up(y.e[e])));
+            }
+            st_vec<T>(p + t * N, x[u]);
+            continue;
+        }
+        size_t i = t - c.nv;
+        if (i >= head) i += c.nv * N;
+        if (i < head + c.nv * N + c.rest / sizeof(T)) acc[i] = Traits<T>::down(op_apply<OP, A>(Traits<T>::up(acc[i]), Traits<T>::up(in[i])));
+    }
 }
 
 cudaError_t launch_local_copy(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
@@ -126,6 +136,15 @@ cudaError_t launch_local_copy(void* dst, const void* src, size_t bytes, cudaStre
     return launch_early(k_local_copy, (unsigned)(grid ? grid : 1), kCopyThreads, stream, (char*)dst, (const char*)src, c);
 }
 
+/**
+ * The shape of a fold of `bytes` per operand. One vector per thread and CTAs of 512 stream best out of HBM; where both operands
+ * can be in L2, its latency counts and two vectors per thread in CTAs of 128 are ahead. Probe of the two shapes, us, operands
+ * of three sets in turn / of sets that come from HBM: 8 MiB 2.75 -> 2.63 / 4.63 -> 4.79, 12 MiB 3.71 -> 3.62 / 6.33 -> 6.14,
+ * 16 MiB 6.95 -> 6.15 / 8.51 -> 8.51, 20 MiB 10.21 -> 9.40 / 10.57 -> 10.55, 22 MiB 11.19 -> 10.61 / 11.45 -> 11.54,
+ * 24 MiB 12.21 -> 12.02 / 12.30 -> 12.44, 28 MiB 14.00 -> 14.16 / 13.97 -> 14.15, 1 GiB 450 -> 457.
+ */
+static bool two_vectors(size_t bytes) { return bytes >= (10u << 20) && bytes <= (22u << 20); }
+
 cudaError_t launch_local_reduce(void* acc, const void* in, size_t count, ncclDataType_t dt, ncclRedOp_t op, cudaStream_t stream) {
     if (!count) return cudaSuccess;
     const size_t es = dt == ncclInt8 || dt == ncclUint8 ? 1 : dt == ncclFloat16 || dt == ncclBfloat16 ? 2
@@ -134,11 +153,12 @@ cudaError_t launch_local_reduce(void* acc, const void* in, size_t count, ncclDat
     // a pairwise fold has no world size: ncclAvg accumulates like ncclSum here
     const Cut c = cut_range(acc, in, count * es);
     const size_t threads = c.nv + (c.head + c.rest) / es;
-    const unsigned grid = (unsigned)((threads + kReduceThreads - 1) / kReduceThreads);
     cudaError_t e = cudaErrorInvalidValue;
-#define CALL(T, OP) e = launch_early(k_local_reduce<T, OP>, grid, kReduceThreads, stream, (T*)acc, (const T*)in, c)
+#define SHAPED(T, OP, THREADS, U) launch_early(k_local_reduce<T, OP, THREADS, U>, (unsigned)((threads + THREADS * U - 1) / (THREADS * U)), THREADS, stream, (T*)acc, (const T*)in, c)
+#define CALL(T, OP) e = two_vectors(count * es) ? SHAPED(T, OP, 128, 2) : SHAPED(T, OP, 512, 1)
     DCCL_DISPATCH_TYPE_OP((int)dt, (int)op, CALL)
 #undef CALL
+#undef SHAPED
     return e;
 }
 

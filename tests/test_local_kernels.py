@@ -68,6 +68,26 @@ def test_fold_at_every_pair_of_offsets(dccl_lib, dtype, op):
                 assert torch.equal(torch.nan_to_num(acc), torch.nan_to_num(want)) and torch.equal(acc.isnan(), want.isnan()), (count, ao, xo)
 
 
+@pytest.mark.parametrize("edge", [10 << 20, 22 << 20])
+@pytest.mark.parametrize("dtype", [torch.int8, torch.bfloat16, torch.float32, torch.float64])
+def test_fold_where_its_shape_changes(dccl_lib, dtype, edge):
+    """Below, at and above the sizes between which a thread folds two vectors; ends of every kind; nothing else is touched."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    es = torch.empty((), dtype=dtype).element_size()
+    stream = torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator(device="cuda").manual_seed(edge)
+    room = edge // es + 8192
+    x = torch.randint(-50, 50, (room,), device="cuda", generator=gen).to(dtype)      # sums of two are exact in every type
+    a = torch.randint(-50, 50, (room,), device="cuda", generator=gen).to(dtype)
+    for count in (edge // es - 1, edge // es, edge // es + 1, edge // es + 4096 // es + 3):
+        for ao, xo in ((0, 0), (0, 3), (1, 0), (3, 1)):
+            acc, want = a.clone(), a.clone()
+            assert dccl_lib.dccl_local_reduce_device(acc[ao:].data_ptr(), x[xo:].data_ptr(), count, dtype_of(acc), OPS["sum"], stream) == 0
+            want[ao:ao + count] += x[xo:xo + count]
+            assert torch.equal(acc, want), (count, ao, xo)
+
+
 def test_fold_into_itself_and_pointers_between_elements(dccl_lib):
     if not torch.cuda.is_available():
         pytest.skip("needs a GPU")
