@@ -3,7 +3,7 @@
  * only kernel, reference src/core/reduce.cu:9-38, as a vectorised, operator-
  * templated grid), and the bounded-wait self test.
  */
-#include "byte_ops.cuh"
+#include "packed_ops.cuh"
 #include "launch_early.cuh"
 #include "kernels.hpp"
 #include "../device/reduce_ops.cuh"
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kCopyThreads) k_local_copy(char* dst, const ch
  * the copy: 1 GiB fp32 takes 446 us (7.2 TB/s), 25 MiB bf16 12.7 us and 1 MiB 3.3 us (the host's cost of the call), where two
  * resident CTAs per SM with eight vectors in flight per thread, each CTA on a piece of at least 64 KB, took 520, 16.4 and 5.1 us.
  * Operands at different distances from a 16-byte boundary read `in` through a window as the copy does: 12 MB of fp16 24.6 ->
- * 4.3 us (before: one element per access). The elements outside the vectors get threads of their own behind the vectors' threads.
+ * 3.9 us (before: one element per access). The elements outside the vectors get threads of their own behind the vectors' threads.
  */
 template <typename T, int OP, int THREADS, int U>
 __global__ void __launch_bounds__(THREADS) k_local_reduce(T* acc, const T* in, const __grid_constant__ Cut c) {
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(THREADS) k_local_reduce(T* acc, const T* in, c
         if (t < c.nv) {
             Vec16<T> y;
             *reinterpret_cast<uint4*>(&y) = cut_out(w[u], c.shift);
-            if constexpr (kFoldsBytes<T, OP>) fold_bytes<T, OP>(x[u], y);
+            if constexpr (kFoldsBytes<T, OP> || kFoldsPairs<T, OP>) fold_packed<T, OP>(x[u], y);
             else {
 #pragma unroll
                 for (int e = 0; e < N; e++) x[u].e[e] = Traits<T>::down(op_apply<OP, A>(Traits<T>::up(x[u].e[e]), Traits<T>::up(y.e[e])));

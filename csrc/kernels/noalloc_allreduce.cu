@@ -6,7 +6,7 @@
  * calls (and outputs that are another rank's input) correct without any ordering between threads.
  */
 #include "noalloc_allreduce.h"
-#include "byte_ops.cuh"
+#include "packed_ops.cuh"
 #include "launch_early.cuh"
 #include "../device/reduce_ops.cuh"
 #include <cstdint>
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kNoAllocThreads) k_noalloc_allreduce(const __g
             A acc[N];
             if constexpr (kFoldsBytes<T, OP>) {
 #pragma unroll
-                for (int k = 1; k < DCCL_NOALLOC_MAX_RANKS; k++) if (k < n) fold_bytes<T, OP>(v[0], v[k]);
+                for (int k = 1; k < DCCL_NOALLOC_MAX_RANKS; k++) if (k < n) fold_packed<T, OP>(v[0], v[k]);
             }
 #pragma unroll
             for (int e = 0; e < N; e++) acc[e] = Traits<T>::up(v[0].e[e]);

@@ -68,6 +68,31 @@ def test_fold_at_every_pair_of_offsets(dccl_lib, dtype, op):
                 assert torch.equal(torch.nan_to_num(acc), torch.nan_to_num(want)) and torch.equal(acc.isnan(), want.isnan()), (count, ao, xo)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("op", ["sum", "max", "min"])
+def test_pairs_of_16_bit_floats_fold_as_they_do_one_by_one(dccl_lib, dtype, op):
+    """Every bit pattern against every 29th one and the special ones, in both orders."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    every = torch.arange(-32768, 32768, device="cuda", dtype=torch.int32).to(torch.int16).view(dtype)
+    some = [0, 1, 0x03FF, 0x0400, 0x7BFF, 0x7C00, 0x7C01, 0x7E00, 0x7F7F, 0x7F80, 0x7F81, 0x7FFF, 0x007F, 0x0080]
+    some = torch.tensor(some + [s - 0x8000 for s in some] + list(range(-32768, 32768, 29)), device="cuda", dtype=torch.int32).to(torch.int16).view(dtype)
+    stream = torch.cuda.current_stream().cuda_stream
+    for part in some.split(256):
+        x = every.repeat(part.numel())
+        a = part.repeat_interleave(every.numel())
+        for first, second in ((a, x), (x, a)):
+            acc, p, q = first.clone(), first.float(), second.float()
+            assert dccl_lib.dccl_local_reduce_device(acc.data_ptr(), second.data_ptr(), acc.numel(), dtype_of(acc), OPS[op], stream) == 0
+            if op == "sum":
+                want = (p + q).to(dtype)
+            else:                                                # of equal values, two zeros among them, the first; a NaN loses to a number
+                want = torch.where(((p < q) if op == "max" else (q < p)) | p.isnan(), second, first)
+            nan = want.isnan()
+            assert torch.equal(acc.isnan(), nan)
+            assert torch.equal(acc.view(torch.int16).masked_fill(nan, 0), want.view(torch.int16).masked_fill(nan, 0))
+
+
 @pytest.mark.parametrize("edge", [10 << 20, 22 << 20])
 @pytest.mark.parametrize("dtype", [torch.int8, torch.bfloat16, torch.float32, torch.float64])
 def test_fold_where_its_shape_changes(dccl_lib, dtype, edge):
