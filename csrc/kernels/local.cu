@@ -59,28 +59,27 @@ static Cut cut_range(const void* dst, const void* src, size_t bytes) {
 
 /**
  * HBM bounds a large copy, launch and latency a small one. Every thread moves two vectors and the CTAs follow each other
- * through memory, so that all SMs work in one window of a few MB: 1 GiB takes 312 us (6.9 TB/s of reads and writes) where
- * two resident CTAs per SM, each on a contiguous piece of its own, took 363 us (296 places of memory open at once). The
- * same shape is within 3 % of the best from 64 KB to 1 GiB (one to four vectors, 256 to 1024 threads, 16- and 32-byte
- * accesses were tried), so there is one. Pointers with different distances to a 16-byte boundary cost a second load, which
- * the L1 cache serves, and a few selects: 26 MB of bf16 from a source 6 bytes off take 9.4 us where a loop over single bytes
- * took 88.2 us.
+ * through memory, so that all SMs work in one window of a few MB: 1 GiB takes 304 us (7.1 TB/s of reads and writes) where
+ * two resident CTAs per SM, each on a contiguous piece of its own, took 363 us (296 places of memory open at once). Pointers
+ * with different distances to a 16-byte boundary cost a second load, which the L1 cache serves, and a few selects: 26 MB of
+ * bf16 from a source 6 bytes off take 9.4 us where a loop over single bytes took 88.2 us.
  */
-constexpr int kCopyThreads = 256, kCopyU = 2;
-__global__ void __launch_bounds__(kCopyThreads) k_local_copy(char* dst, const char* src, const __grid_constant__ Cut c) {
+constexpr int kCopyU = 2;
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_local_copy(char* dst, const char* src, const __grid_constant__ Cut c) {
     wait_for_stream();
-    const size_t i0 = (size_t)blockIdx.x * (kCopyThreads * kCopyU) + threadIdx.x;
+    const size_t i0 = (size_t)blockIdx.x * (THREADS * kCopyU) + threadIdx.x;
     const char* q = src + c.head - c.shift;
     Window w[kCopyU];
 #pragma unroll
     for (int u = 0; u < kCopyU; u++)
-        if (i0 + u * kCopyThreads < c.nv) load(w[u], q + (i0 + u * kCopyThreads) * 16, c.shift);
+        if (i0 + u * THREADS < c.nv) load(w[u], q + (i0 + u * THREADS) * 16, c.shift);
 #pragma unroll
     for (int u = 0; u < kCopyU; u++)
-        if (i0 + u * kCopyThreads < c.nv) *reinterpret_cast<uint4*>(dst + c.head + (i0 + u * kCopyThreads) * 16) = cut_out(w[u], c.shift);
+        if (i0 + u * THREADS < c.nv) *reinterpret_cast<uint4*>(dst + c.head + (i0 + u * THREADS) * 16) = cut_out(w[u], c.shift);
     if (blockIdx.x == 0) {      // at most 30 bytes before and 30 behind the vectors
-        for (size_t j = threadIdx.x; j < c.head; j += kCopyThreads) dst[j] = src[j];
-        for (size_t j = c.head + c.nv * 16 + threadIdx.x; j < c.head + c.nv * 16 + c.rest; j += kCopyThreads) dst[j] = src[j];
+        for (size_t j = threadIdx.x; j < c.head; j += THREADS) dst[j] = src[j];
+        for (size_t j = c.head + c.nv * 16 + threadIdx.x; j < c.head + c.nv * 16 + c.rest; j += THREADS) dst[j] = src[j];
     }
 }
 
@@ -132,8 +131,12 @@ __global__ void __launch_bounds__(THREADS) k_local_reduce(T* acc, const T* in, c
 cudaError_t launch_local_copy(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
     if (!bytes || dst == src) return cudaSuccess;
     const Cut c = cut_range(dst, src, bytes);
-    const size_t per = (size_t)kCopyThreads * kCopyU, grid = (c.nv + per - 1) / per;
-    return launch_early(k_local_copy, (unsigned)(grid ? grid : 1), kCopyThreads, stream, (char*)dst, (const char*)src, c);
+    // CTAs of 1024 threads once a copy streams out of HBM, of 256 before: probe of the two, us, 20 MiB 7.46 / 7.18, 24 MiB
+    // 8.74 / 8.73, 28 MiB 9.99 / 10.15, 32 MiB 11.18 / 11.35, 64 MiB 20.82 / 21.07, 1 GiB 305 / 309; 25 MiB from a source 6
+    // bytes off 9.52 / 9.40
+    const unsigned threads = bytes >= (28u << 20) ? 1024 : 256;
+    const size_t per = (size_t)threads * kCopyU, grid = (c.nv + per - 1) / per;
+    return launch_early(threads == 1024 ? k_local_copy<1024> : k_local_copy<256>, (unsigned)(grid ? grid : 1), threads, stream, (char*)dst, (const char*)src, c);
 }
 
 /**

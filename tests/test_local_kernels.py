@@ -38,6 +38,16 @@ def test_copy_at_every_pair_of_offsets(comm, nbytes):
             assert torch.equal(dst, want), (nbytes, so, do)
 
 
+@pytest.mark.parametrize("nbytes", [(28 << 20) - 1, 28 << 20, (28 << 20) + 32768 + 17])
+def test_copy_where_its_shape_changes(comm, nbytes):
+    src = torch.randint(0, 255, (nbytes + 32,), dtype=torch.uint8, device="cuda", generator=torch.Generator(device="cuda").manual_seed(nbytes))
+    for so, do in ((0, 0), (6, 0), (0, 1), (3, 13)):
+        dst = torch.full((nbytes + 32,), 0xAB, dtype=torch.uint8, device="cuda")
+        comm.all_gather(src[so:so + nbytes], dst[do:do + nbytes])
+        assert torch.equal(dst[do:do + nbytes], src[so:so + nbytes])
+        assert bool((dst[:do] == 0xAB).all()) and bool((dst[do + nbytes:] == 0xAB).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.int8, torch.uint8, torch.int32, torch.int64, torch.float16, torch.bfloat16, torch.float32, torch.float64])
 @pytest.mark.parametrize("op", ["sum", "prod", "max", "min"])
 def test_fold_at_every_pair_of_offsets(dccl_lib, dtype, op):
