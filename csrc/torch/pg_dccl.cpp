@@ -24,6 +24,7 @@
 
 #define DCCL_WITH_CUDA_RUNTIME 1
 #include <dccl/dccl.hpp>
+#include "adamw_step.hpp"
 
 #include <atomic>
 #include <cstring>
@@ -446,7 +447,8 @@ private:
 } // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
-    m.doc() = "PyTorch process-group backend of the DCCL B200 collective library";
+    m.doc() = "PyTorch process-group backend of the DCCL B200 collective library, and the host side of its AdamW update";
+    if (add_adamw_step(m.ptr()) != 0) throw pybind11::error_already_set();
     m.def("create_backend", &BackendDccl::create, "create a c10d backend over a store");
     m.def("comm_handle", [](const c10::intrusive_ptr<c10d::Backend>& b) -> uintptr_t {
         auto* d = dynamic_cast<BackendDccl*>(b.get());

@@ -1,9 +1,11 @@
-"""Builds the PyTorch backend extension (csrc/torch/pg_dccl.cpp) in-tree, next to libdccl.so.
+"""Builds the PyTorch extension (csrc/torch: the process-group backend and the host side of the AdamW update) in-tree, next to
+libdccl.so, and loads it.
 
 The extension only uses the library's public C++ API and libtorch; it is compiled with the system
 C++ compiler against the headers of the installed torch and linked to ``dccl_b200/lib/libdccl.so``
 by relative rpath, so the built file can be moved with the package.
 """
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -13,14 +15,15 @@ import sysconfig
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _PKG = os.path.dirname(_HERE)
 _ROOT = os.path.dirname(_PKG)
-SRC = os.path.join(_ROOT, "csrc", "torch", "pg_dccl.cpp")
+SRC_DIR = os.path.join(_ROOT, "csrc", "torch")
+SRCS = [os.path.join(SRC_DIR, name) for name in ("pg_dccl.cpp", "adamw_step.cpp")]
 OUT = os.path.join(_PKG, "lib", "_dccl_torch.so")
 
 
 def needs_build():
     if not os.path.exists(OUT):
         return True
-    newest = max(os.path.getmtime(SRC), os.path.getmtime(os.path.join(_ROOT, "include", "dccl", "dccl.hpp")))
+    newest = max(os.path.getmtime(f) for f in SRCS + [os.path.join(SRC_DIR, "adamw_step.hpp"), os.path.join(_ROOT, "include", "dccl", "dccl.hpp")])
     return os.path.getmtime(OUT) < newest
 
 
@@ -36,7 +39,7 @@ def build(force=False, verbose=False):
     tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
     incs = cpp_extension.include_paths(device_type="cuda")
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", SRC, "-o", OUT,
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", *SRCS, "-o", OUT,
            "-DTORCH_EXTENSION_NAME=_dccl_torch", "-DTORCH_API_INCLUDE_EXTENSION_H", "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
            "-I" + os.path.join(_ROOT, "include"), "-I" + os.path.join(cuda_home, "include"), "-I" + sysconfig.get_paths()["include"]]
     cmd += ["-I" + p for p in incs]
@@ -49,6 +52,20 @@ def build(force=False, verbose=False):
     if verbose:
         print(res.stderr, file=sys.stderr)
     return OUT
+
+
+_module = None
+
+
+def load():
+    """The extension module (built on first use when it is missing or older than its sources)."""
+    global _module
+    if _module is None:
+        spec = importlib.util.spec_from_file_location("_dccl_torch", build())
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _module = module
+    return _module
 
 
 if __name__ == "__main__":

@@ -8,26 +8,15 @@ kernels (see csrc/torch/pg_dccl.cpp). ``communicator(pg)`` returns a
 ``dccl_b200.Communicator`` that shares the process group's native
 communicator, e.g. for symmetric allocations or for choosing a variant.
 """
-import importlib.util
-
 import torch
 import torch.distributed as dist
 
 from . import backend_build
 
-_ext = None
-
 
 def extension():
     """The compiled backend module (built in-tree on first use)."""
-    global _ext
-    if _ext is None:
-        path = backend_build.build()
-        spec = importlib.util.spec_from_file_location("_dccl_torch", path)
-        mod = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(mod)
-        _ext = mod
-    return _ext
+    return backend_build.load()
 
 
 def _create(store, rank, size, timeout):

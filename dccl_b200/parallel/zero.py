@@ -18,8 +18,8 @@ symmetric memory (``symmetric=True``), so that both collectives run zero-copy th
 ``close()`` before the communicator is finalized to give that memory back.
 """
 import ctypes
-import math
 import os
+import warnings
 
 import torch
 import torch.optim.adam as _adam
@@ -27,9 +27,9 @@ import torch.optim.optimizer as _optimizer
 from torch.utils._device import DeviceContext
 
 from .._lib import lib
-from ..comm import DcclError, current_stream_handle, dtype_of
+from ..comm import DcclError
+from . import backend_build
 
-_FUSED_DTYPES = (torch.bfloat16, torch.float16, torch.float32)
 _IN_OPTIMIZER, _IN_ADAM = vars(_optimizer), vars(_adam)
 _enter_range, _exit_range = torch._C._autograd._record_function_with_args_enter, torch._C._autograd._record_function_with_args_exit
 
@@ -46,6 +46,22 @@ def _observer_query():
 
 
 _observed = _observer_query()
+
+_native = None
+
+
+def _native_step():
+    """(check, update, address of the launch) of the host side of the one-kernel update (csrc/torch/adamw_step.cpp), or () where
+    the extension that holds it can neither be loaded nor built: torch's own step runs then."""
+    global _native
+    if _native is None:
+        try:
+            ext = backend_build.load()
+            _native = ext.adamw_ready, ext.adamw_update, ctypes.cast(lib().dccl_adamw_flat, ctypes.c_void_p).value
+        except (ImportError, OSError, RuntimeError, AttributeError) as e:
+            warnings.warn("dccl_b200: AdamW steps of sharded optimizers run as torch's own, several times slower than as one kernel: %s" % e)
+            _native = ()
+    return _native
 
 
 def _step_is_torchs_own():
@@ -110,6 +126,8 @@ class ShardedOptimizer:
                                 "grad_slice": torch.empty(per, dtype=dtype, device=device),
                                 "out_slice": torch.empty(per, dtype=dtype, device=device)})
         self.inner = optimizer_cls(masters, **kwargs)
+        if optimizer_cls is torch.optim.AdamW and any(m.is_cuda for m in masters):
+            _native_step()
 
     def zero_grad(self):
         for g in self.groups:
@@ -152,26 +170,15 @@ class ShardedOptimizer:
             return None
         if len(inner.param_groups) != 1 or len(inner.param_groups[0]["params"]) != len(self.groups):
             return None
-        o = inner.param_groups[0]
-        if o["amsgrad"] or o["maximize"] or o["capturable"] or o["differentiable"] or o["fused"] or not o.get("decoupled_weight_decay", True):
+        if not self.groups[0]["master"].is_cuda or not _native_step():
             return None
-        for x in (o["lr"], o["weight_decay"], o["eps"], *o["betas"]):
-            if not isinstance(x, (int, float)):
-                return None
-        updates = []
+        ready, o, updates = _native[0], inner.param_groups[0], []
         for g, p in zip(self.groups, o["params"]):
+            # options of plain AdamW, state on the GPU as the kernel reads it, and no capture
             st = inner.state.get(p)
-            if p is not g["master"] or not p.is_cuda or not st or g["grad"].dtype not in _FUSED_DTYPES:
+            if p is not g["master"] or not st or not ready(o, st, p, p.grad, g["grad"], g["per"]):
                 return None
-            step_count, device, per = st.get("step"), p.get_device(), g["per"]
-            if not isinstance(step_count, torch.Tensor) or step_count.is_cuda:
-                return None
-            for t in (p, p.grad, st.get("exp_avg"), st.get("exp_avg_sq")):
-                if type(t) is not torch.Tensor or t.dtype is not torch.float32 or t.get_device() != device or t.numel() != per or not t.is_contiguous():
-                    return None
             updates.append((g, o, st))
-        if torch.cuda.is_current_stream_capturing():
-            return None
         if step is not None:
             inner._opt_called = True
         return updates
@@ -190,18 +197,10 @@ class ShardedOptimizer:
                 _exit_range(entered)
 
     def _adamw(self, g, o, st):
-        p, n = g["master"], self.comm.world
-        device = p.get_device()
-        grad, out = (g["grad_slice"], g["out_slice"]) if n > 1 else (g["grad"], g["flat"])
-        m, v = st["exp_avg"], st["exp_avg_sq"]
-        t, (b1, b2) = st["step"].item() + 1, o["betas"]
-        st["step"].fill_(t)
-        rc = lib().dccl_adamw_flat(device, dtype_of(grad), g["per"], p.data_ptr(), p.grad.data_ptr(), m.data_ptr(), v.data_ptr(),
-                                   grad.data_ptr(), out.data_ptr(), 1 - o["lr"] * o["weight_decay"], 1 - b1, b2, 1 - b2,
-                                   o["lr"] / (1 - b1 ** t), math.sqrt(1 - b2 ** t), o["eps"], current_stream_handle(device))
-        if rc != 0:
+        p = g["master"]
+        grad, out = (g["grad_slice"], g["out_slice"]) if self.comm.world > 1 else (g["grad"], g["flat"])
+        if _native[1](_native[2], o, st, p, p.grad, grad, out, g["per"]) != 0:
             raise DcclError(1, "AdamW update")
-        torch.autograd.graph.increment_version((p, p.grad, m, v, out))
 
     def close(self):
         """Give symmetric buffers back (collective). The parameters keep their values in ordinary memory."""

@@ -362,6 +362,61 @@ def test_options_and_state_the_kernel_does_not_take(cuda_lib, monkeypatch, chang
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("kind", [lambda s: s.double(), lambda s: s.reshape(1), lambda s: s.long(), lambda s: torch.nn.Parameter(s, requires_grad=False)],
+                         ids=["fp64", "one element", "integer", "subclass"])
+def test_step_counts_of_other_kinds_are_counted_in_place(cuda_lib, monkeypatch, kind):
+    a, b = _stepped(False), _stepped(True)
+    _state("step", kind)(a, monkeypatch)                        # torch's own step does not take all of these
+    assert a._adamw_updates() is not None
+    count = a.inner.state[a.groups[0]["master"]]["step"]
+    version = count._version
+    a, b = _train(a, 2), _train(b, 2)
+    assert a.inner.state[a.groups[0]["master"]]["step"] is count and count.item() == 3 and count._version == version + 2
+    torch.testing.assert_close(a.groups[0]["master"], b.groups[0]["master"], rtol=3 * 2.0 ** -23, atol=1e-7)
+
+
+@pytest.mark.gpu
+def test_a_step_count_that_torch_refuses_to_change(cuda_lib):
+    opt = _stepped(False)
+    st, before = opt.inner.state[opt.groups[0]["master"]], opt.groups[0]["flat"].clone()
+    with torch.inference_mode():
+        st["step"] = st["step"].clone()
+    with pytest.raises(RuntimeError, match="[Ii]nference"):
+        opt.step()
+    assert torch.equal(opt.groups[0]["flat"], before)
+
+
+@pytest.mark.gpu
+def test_what_a_step_changes_is_a_new_version(cuda_lib):
+    opt = _stepped(False)
+    g, st = opt.groups[0], opt.inner.state[opt.groups[0]["master"]]
+    changed = (g["master"], g["master"].grad, st["exp_avg"], st["exp_avg_sq"], st["step"], g["flat"])
+    before = [x._version for x in changed] + [g["grad"]._version]
+    opt.step()
+    assert [x._version for x in changed] + [g["grad"]._version] == [v + 1 for v in before[:-1]] + before[-1:]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("betas,taken", [([0.9, 0.95], True), ((0, 0.95), True), ((1.0, 0.95), False), ((0.9, 1.0), False), ((-0.1, 0.95), False),
+                                         ((0.9, float("nan")), False), ((0.9,), False), ((0.9, "0.95"), False)])
+def test_betas_the_kernel_takes(cuda_lib, betas, taken):
+    opt = _stepped(False)
+    opt.inner.param_groups[0]["betas"] = betas
+    assert (opt._adamw_updates() is not None) == taken
+
+
+def test_without_the_extension_torch_steps(monkeypatch):
+    def broken():
+        raise RuntimeError("no compiler")
+
+    monkeypatch.setattr(zero, "_native", None)
+    monkeypatch.setattr(zero.backend_build, "load", broken)
+    with pytest.warns(UserWarning, match="no compiler"):
+        assert zero._native_step() == ()
+    assert zero._native_step() == ()                            # said once
+
+
+@pytest.mark.gpu
 def test_optimizers_dtypes_and_surroundings_the_kernel_does_not_take(cuda_lib, monkeypatch):
     assert _stepped(False, cls=torch.optim.Adam)._adamw_updates() is None
     assert _stepped(False, cls=type("Derived", (torch.optim.AdamW,), {}))._adamw_updates() is None
