@@ -23,8 +23,9 @@ OUT = os.path.join(_PKG, "lib", "_dccl_torch.so")
 def needs_build():
     if not os.path.exists(OUT):
         return True
-    newest = max(os.path.getmtime(f) for f in SRCS + [os.path.join(SRC_DIR, "adamw_step.hpp"), os.path.join(_ROOT, "include", "dccl", "dccl.hpp")])
-    return os.path.getmtime(OUT) < newest
+    sources = SRCS + [os.path.join(SRC_DIR, "adamw_step.hpp"), os.path.join(_ROOT, "include", "dccl", "dccl.hpp")]
+    # a package that came without its sources is as new as it gets
+    return any(os.path.exists(f) and os.path.getmtime(OUT) < os.path.getmtime(f) for f in sources)
 
 
 def build(force=False, verbose=False):
@@ -39,7 +40,8 @@ def build(force=False, verbose=False):
     tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
     incs = cpp_extension.include_paths(device_type="cuda")
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", *SRCS, "-o", OUT,
+    part = "%s.%d" % (OUT, os.getpid())      # ranks that build at the same time do not write into each other's file
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", *SRCS, "-o", part,
            "-DTORCH_EXTENSION_NAME=_dccl_torch", "-DTORCH_API_INCLUDE_EXTENSION_H", "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
            "-I" + os.path.join(_ROOT, "include"), "-I" + os.path.join(cuda_home, "include"), "-I" + sysconfig.get_paths()["include"]]
     cmd += ["-I" + p for p in incs]
@@ -49,6 +51,7 @@ def build(force=False, verbose=False):
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("building the torch backend failed:\n" + " ".join(cmd) + "\n" + res.stderr[-6000:])
+    os.replace(part, OUT)
     if verbose:
         print(res.stderr, file=sys.stderr)
     return OUT
