@@ -62,6 +62,20 @@ bool read_options(PyObject* group, Options* o) {
            && o->beta1 >= 0 && o->beta1 < 1 && o->beta2 >= 0 && o->beta2 < 1;
 }
 
+/** A step count in plain memory of the host, which is read and changed in place. Anything else (another type, a subclass, an
+ *  inference tensor, which torch may refuse to change) goes through torch. */
+bool counts_in_place(PyObject* count, const at::Tensor& t) {
+    return is_plain_tensor(count) && t.scalar_type() == at::kFloat && t.is_cpu() && t.numel() == 1 && t.layout() == at::kStrided
+           && !t.is_inference() && !t.requires_grad() && !t.is_neg();
+}
+
+/** A step count of zero or more. Below zero the bias corrections divide by zero or have no square root, which torch's step reports. */
+bool counts_up(PyObject* count) {
+    const at::Tensor t = THPVariable_Unpack(count);
+    if (t.numel() != 1 || t.is_complex()) return false;
+    return (counts_in_place(count, t) ? (double)*t.const_data_ptr<float>() : t.item().toDouble()) >= 0;
+}
+
 /** adamw_ready(param_group, state, master, master_grad, grad, n): whether the kernel can update this slice of n elements, now that
  *  nothing is being captured. */
 PyObject* adamw_ready(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
@@ -75,19 +89,17 @@ PyObject* adamw_ready(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const c10::Device device = THPVariable_Unpack(args[2]).device();
     if (!device.is_cuda() || flat_dtype(THPVariable_Unpack(args[4]).scalar_type()) < 0 || !read_options(group, &o)) Py_RETURN_FALSE;
     PyObject* count = PyDict_GetItem(state, key.step);
-    if (!count || !THPVariable_Check(count) || THPVariable_Unpack(count).is_cuda()) Py_RETURN_FALSE;
+    if (!count || !THPVariable_Check(count) || THPVariable_Unpack(count).is_cuda() || !counts_up(count)) Py_RETURN_FALSE;
     for (PyObject* t : {args[2], args[3], PyDict_GetItem(state, key.exp_avg), PyDict_GetItem(state, key.exp_avg_sq)})
         if (!is_flat_fp32(t, n, device)) Py_RETURN_FALSE;
     return PyBool_FromLong(c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None);
     END_HANDLE_TH_ERRORS
 }
 
-/** Counts the step and returns its number. A plain fp32 scalar on the host is changed in place; anything else (another type, a
- *  subclass, an inference tensor, which torch may refuse to change) goes through torch. */
+/** Counts the step and returns its number. */
 double next_step(PyObject* count) {
     const at::Tensor t = THPVariable_Unpack(count);
-    if (is_plain_tensor(count) && t.scalar_type() == at::kFloat && t.is_cpu() && t.numel() == 1 && t.layout() == at::kStrided
-        && !t.is_inference() && !t.requires_grad() && !t.is_neg()) {
+    if (counts_in_place(count, t)) {
         float* p = t.mutable_data_ptr<float>();
         const double now = (double)*p + 1;
         *p = (float)now;

@@ -387,6 +387,21 @@ def test_a_step_count_that_torch_refuses_to_change(cuda_lib):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("count", [-1.0, -0.5, -3.0, float("-inf")])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_step_counts_below_zero_are_torchs_to_report(cuda_lib, monkeypatch, count, dtype):
+    a, b = _stepped(False), _stepped(True)
+    for opt in (a, b):
+        _state("step", lambda s: torch.tensor(count, dtype=dtype))(opt, monkeypatch)
+    assert a._adamw_updates() is None
+    if count == -1:
+        for opt in (a, b):
+            with pytest.raises(ZeroDivisionError):
+                opt.step()
+        assert torch.equal(a.groups[0]["flat"], b.groups[0]["flat"]) and torch.isfinite(a.groups[0]["flat"]).all()
+
+
+@pytest.mark.gpu
 def test_what_a_step_changes_is_a_new_version(cuda_lib):
     opt = _stepped(False)
     g, st = opt.groups[0], opt.inner.state[opt.groups[0]["master"]]
