@@ -8,6 +8,7 @@
 #include "adamw_step.hpp"
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -43,22 +44,31 @@ bool number(PyObject* o, double* v) {
     return true;
 }
 
+/** Whether Python takes `o` for true; what has no truth value, and a missing option, is left to torch to report (-1). */
+int truth(PyObject* o) {
+    if (o == Py_False || o == Py_None) return 0;
+    if (!o) return -1;
+    const int t = PyObject_IsTrue(o);
+    if (t < 0) PyErr_Clear();
+    return t;
+}
+
 struct Options { double lr, weight_decay, eps, beta1, beta2; };
 
 /** The options of a parameter group, when they are those of plain AdamW. Betas outside [0, 1), which torch refuses or fails on,
  *  are left to it. */
 bool read_options(PyObject* group, Options* o) {
-    for (PyObject* k : {key.amsgrad, key.maximize, key.capturable, key.differentiable, key.fused}) {
-        PyObject* flag = PyDict_GetItem(group, k);
-        if (flag != Py_False && flag != Py_None) return false;
-    }
+    for (PyObject* k : {key.amsgrad, key.maximize, key.capturable, key.differentiable, key.fused})
+        if (truth(PyDict_GetItem(group, k)) != 0) return false;
     PyObject* decoupled = PyDict_GetItem(group, key.decoupled_weight_decay);
-    if (decoupled && decoupled != Py_True) return false;
+    if (decoupled && truth(decoupled) != 1) return false;
     PyObject* betas = PyDict_GetItem(group, key.betas);
-    if (!betas || !(PyTuple_Check(betas) || PyList_Check(betas)) || PySequence_Fast_GET_SIZE(betas) != 2) return false;
-    return number(PyDict_GetItem(group, key.lr), &o->lr) && number(PyDict_GetItem(group, key.weight_decay), &o->weight_decay)
+    const THPObjectPtr pair(betas ? PySequence_Fast(betas, "") : nullptr);     // any two numbers in a row: an array, a list of a configuration file
+    if (!pair) { PyErr_Clear(); return false; }
+    return PySequence_Fast_GET_SIZE(pair.get()) == 2
+           && number(PyDict_GetItem(group, key.lr), &o->lr) && number(PyDict_GetItem(group, key.weight_decay), &o->weight_decay)
            && number(PyDict_GetItem(group, key.eps), &o->eps)
-           && number(PySequence_Fast_GET_ITEM(betas, 0), &o->beta1) && number(PySequence_Fast_GET_ITEM(betas, 1), &o->beta2)
+           && number(PySequence_Fast_GET_ITEM(pair.get(), 0), &o->beta1) && number(PySequence_Fast_GET_ITEM(pair.get(), 1), &o->beta2)
            && o->beta1 >= 0 && o->beta1 < 1 && o->beta2 >= 0 && o->beta2 < 1;
 }
 

@@ -1,8 +1,10 @@
 """The one-kernel AdamW update of dccl_b200.parallel.zero against the general path (torch's own optimizer and the casts
 around it), and which optimizers may take it."""
+import collections
 import functools
 import warnings
 
+import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -429,6 +431,27 @@ def test_without_the_extension_torch_steps(monkeypatch):
     with pytest.warns(UserWarning, match="no compiler"):
         assert zero._native_step() == ()
     assert zero._native_step() == ()                            # said once
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,value", [("amsgrad", 0), ("maximize", np.False_), ("fused", 0), ("decoupled_weight_decay", 1), ("betas", np.array([0.9, 0.95])),
+                                        ("betas", collections.deque([0.9, 0.95])), ("betas", collections.UserList([0.9, 0.95])), ("lr", np.float64(1e-2)), ("eps", 0)])
+def test_options_that_python_takes_for_plain_ones(cuda_lib, monkeypatch, name, value):
+    a, b = _stepped(False), _stepped(False)
+    _option(name, lambda: value)(a, monkeypatch)
+    if name == "eps":
+        b.inner.param_groups[0]["eps"] = 0.0
+    assert a._adamw_updates() is not None
+    _same_after_a_step(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,value", [("amsgrad", 1), ("maximize", torch.ones(2, dtype=torch.bool)), ("decoupled_weight_decay", 0), ("betas", np.array([0.9])),
+                                        ("betas", 0.9), ("betas", np.array([0.9, 0.95], dtype=np.float32)), ("betas", collections.deque([0.9, 0.95, 0.99]))])
+def test_options_that_python_takes_for_others(cuda_lib, monkeypatch, name, value):
+    opt = _stepped(False)
+    _option(name, lambda: value)(opt, monkeypatch)
+    assert opt._adamw_updates() is None
 
 
 @pytest.mark.gpu
