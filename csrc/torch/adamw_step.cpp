@@ -47,6 +47,7 @@ bool number(PyObject* o, double* v) {
 /** Whether Python takes `o` for true; what has no truth value, and a missing option, is left to torch to report (-1). */
 int truth(PyObject* o) {
     if (o == Py_False || o == Py_None) return 0;
+    if (o == Py_True) return 1;
     if (!o) return -1;
     const int t = PyObject_IsTrue(o);
     if (t < 0) PyErr_Clear();

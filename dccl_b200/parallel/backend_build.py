@@ -60,11 +60,15 @@ def build(force=False, verbose=False):
 _module = None
 
 
-def load():
-    """The extension module (built on first use when it is missing or older than its sources)."""
+def load(compile=False):
+    """The extension module. A file that is missing or older than its sources is compiled first, or an ImportError."""
     global _module
     if _module is None:
-        spec = importlib.util.spec_from_file_location("_dccl_torch", build())
+        if compile:
+            build()
+        elif needs_build():
+            raise ImportError("%s is missing or older than its sources (python -m dccl_b200.parallel.backend_build builds it)" % OUT)
+        spec = importlib.util.spec_from_file_location("_dccl_torch", OUT)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
         _module = module

@@ -16,7 +16,7 @@ from . import backend_build
 
 def extension():
     """The compiled backend module (built in-tree on first use)."""
-    return backend_build.load()
+    return backend_build.load(compile=True)
 
 
 def _create(store, rank, size, timeout):

@@ -18,6 +18,7 @@ symmetric memory (``symmetric=True``), so that both collectives run zero-copy th
 ``close()`` before the communicator is finalized to give that memory back.
 """
 import ctypes
+import math
 import os
 import warnings
 
@@ -27,9 +28,10 @@ import torch.optim.optimizer as _optimizer
 from torch.utils._device import DeviceContext
 
 from .._lib import lib
-from ..comm import DcclError
+from ..comm import DcclError, current_stream_handle, dtype_of
 from . import backend_build
 
+_FUSED_DTYPES = (torch.bfloat16, torch.float16, torch.float32)
 _IN_OPTIMIZER, _IN_ADAM = vars(_optimizer), vars(_adam)
 _enter_range, _exit_range = torch._C._autograd._record_function_with_args_enter, torch._C._autograd._record_function_with_args_exit
 
@@ -52,16 +54,59 @@ _native = None
 
 def _native_step():
     """(check, update, address of the launch) of the host side of the one-kernel update (csrc/torch/adamw_step.cpp), or () where
-    the extension that holds it can neither be loaded nor built: torch's own step runs then."""
+    the extension that holds it has not been built or cannot be loaded: _adamw_ready and _adamw_update do the same then."""
     global _native
     if _native is None:
         try:
             ext = backend_build.load()
             _native = ext.adamw_ready, ext.adamw_update, ctypes.cast(lib().dccl_adamw_flat, ctypes.c_void_p).value
         except (ImportError, OSError, RuntimeError, AttributeError) as e:
-            warnings.warn("dccl_b200: AdamW steps of sharded optimizers run as torch's own, several times slower than as one kernel: %s" % e)
+            warnings.warn("dccl_b200: the host side of sharded AdamW steps runs in Python, which counts for small models: %s" % e)
             _native = ()
     return _native
+
+
+def _adamw_ready(o, st, p, p_grad, grad, n):
+    """adamw_ready of csrc/torch/adamw_step.cpp, with the same answers."""
+    try:
+        if o["amsgrad"] or o["maximize"] or o["capturable"] or o["differentiable"] or o["fused"] or not o.get("decoupled_weight_decay", True):
+            return False
+        lr, decay, eps, (b1, b2) = o["lr"], o["weight_decay"], o["eps"], o["betas"]
+        for x in (lr, decay, eps, b1, b2):
+            if not isinstance(x, (int, float)):
+                return False
+        if not (0 <= b1 < 1 and 0 <= b2 < 1):
+            return False
+        lr + decay + eps + 0.0
+    except Exception:       # missing, without a truth value, no pair, an integer beyond any float: torch's step reports it
+        return False
+    count, device = st.get("step"), p.get_device()
+    if device < 0 or type(grad) is not torch.Tensor or grad.dtype not in _FUSED_DTYPES or not isinstance(count, torch.Tensor) or count.is_cuda:
+        return False
+    # below zero the bias corrections divide by zero or have no square root, which torch's step reports
+    if count.numel() != 1 or count.is_complex() or not count.item() >= 0:
+        return False
+    for t in (p, p_grad, st.get("exp_avg"), st.get("exp_avg_sq")):
+        if type(t) is not torch.Tensor or t.dtype is not torch.float32 or t.get_device() != device or t.numel() != n or not t.is_contiguous():
+            return False
+    return not torch.cuda.is_current_stream_capturing()
+
+
+def _adamw_update(_, o, st, p, p_grad, grad, out, n):
+    """adamw_update of csrc/torch/adamw_step.cpp. From Python a step of 0.4 M parameters takes 12.8 us, from the extension 5.6."""
+    device, m, v = p.get_device(), st["exp_avg"], st["exp_avg_sq"]
+    count, lr, (b1, b2) = st["step"], o["lr"], o["betas"]
+    t = count.item() + 1
+    count.fill_(t)
+    rc = lib().dccl_adamw_flat(device, dtype_of(grad), n, p.data_ptr(), p_grad.data_ptr(), m.data_ptr(), v.data_ptr(), grad.data_ptr(), out.data_ptr(),
+                               1 - lr * o["weight_decay"], 1 - b1, b2, 1 - b2, lr / (1 - b1 ** t), math.sqrt(1 - b2 ** t), o["eps"],
+                               current_stream_handle(device))
+    if rc == 0:
+        torch.autograd.graph.increment_version((p, p_grad, m, v, out))
+    return rc
+
+
+_IN_PYTHON = _adamw_ready, _adamw_update, None
 
 
 def _step_is_torchs_own():
@@ -170,9 +215,9 @@ class ShardedOptimizer:
             return None
         if len(inner.param_groups) != 1 or len(inner.param_groups[0]["params"]) != len(self.groups):
             return None
-        if not self.groups[0]["master"].is_cuda or not _native_step():
+        if not self.groups[0]["master"].is_cuda:
             return None
-        ready, o, updates = _native[0], inner.param_groups[0], []
+        ready, o, updates = (_native_step() or _IN_PYTHON)[0], inner.param_groups[0], []
         for g, p in zip(self.groups, o["params"]):
             # options of plain AdamW, state on the GPU as the kernel reads it, and no capture
             st = inner.state.get(p)
@@ -199,7 +244,8 @@ class ShardedOptimizer:
     def _adamw(self, g, o, st):
         p = g["master"]
         grad, out = (g["grad_slice"], g["out_slice"]) if self.comm.world > 1 else (g["grad"], g["flat"])
-        if _native[1](_native[2], o, st, p, p.grad, grad, out, g["per"]) != 0:
+        _, update, launch = _native or _IN_PYTHON
+        if update(launch, o, st, p, p.grad, grad, out, g["per"]) != 0:
             raise DcclError(1, "AdamW update")
 
     def close(self):

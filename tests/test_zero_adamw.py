@@ -454,6 +454,70 @@ def test_options_that_python_takes_for_others(cuda_lib, monkeypatch, name, value
     assert opt._adamw_updates() is None
 
 
+def test_the_extension_is_loaded_without_a_compiler_or_not_at_all(monkeypatch, tmp_path):
+    """What an optimizer does while it is made: no rank of a job compiles for a minute there."""
+    monkeypatch.setattr(zero.backend_build, "_module", None)
+    monkeypatch.setattr(zero.backend_build, "OUT", str(tmp_path / "missing.so"))
+    monkeypatch.setattr(zero.backend_build.subprocess, "run", lambda *a, **kw: pytest.fail("a compiler is run"))
+    with pytest.raises(ImportError, match="missing.so"):
+        zero.backend_build.load()
+    monkeypatch.setattr(zero, "_native", None)
+    with pytest.warns(UserWarning, match="missing.so"):
+        assert zero._native_step() == ()
+
+
+@pytest.fixture
+def no_extension(cuda_lib, monkeypatch):
+    def missing():
+        raise ImportError("no extension")
+
+    monkeypatch.setattr(zero, "_native", None)
+    monkeypatch.setattr(zero.backend_build, "load", missing)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("world", [1, 2])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_an_optimizer_without_the_extension_steps_as_one_kernel(dccl_lib, no_extension, monkeypatch, world, dtype):
+    outs = []
+    for extension in (False, True):
+        if extension:
+            monkeypatch.undo()
+            opt = _make(world, dtype, [2049, 7], False)
+        else:
+            with pytest.warns(UserWarning, match="no extension"):
+                opt = _make(world, dtype, [2049, 7], False)
+        _train(opt, 1)
+        general = []
+        opt.inner._optimizer_step_code = lambda: general.append(opt._adamw_updates())
+        _train(opt, 3)
+        assert len(general) == 3 and None not in general and (zero._native != ()) == extension
+        g = opt.groups[0]
+        st = opt.inner.state[g["master"]]
+        outs.append([g["master"], g["master"].grad, g["flat"], st["exp_avg"], st["exp_avg_sq"], st["step"]])
+        assert [x._version for x in outs[-1]] == [x._version for x in outs[0]]
+    assert all(torch.equal(x, y) for x, y in zip(*outs))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("change", [
+    _option("lr", 1), _option("amsgrad", 0), _option("amsgrad", 1), _option("maximize", torch.ones(2, dtype=torch.bool)), _option("capturable", True),
+    _option("differentiable", True), _option("fused", True), _option("decoupled_weight_decay", 0), _option("betas", (1.0, 0.95)), _option("betas", (0.9, float("nan"))),
+    _option("betas", (0.9,)), _option("betas", 0.9), _option("betas", (0.9, "0.95")), _option("betas", np.array([0.9, 0.95])), _option("betas", (0, 0.95)),
+    _option("eps", 10 ** 400), _option("eps", lambda: torch.tensor(1e-8)), _option("weight_decay", None),
+    _state("step", float), _state("step", lambda x: x.cuda()), _state("step", lambda x: -x - 0.5), _state("step", lambda x: x.double()), _state("step", lambda x: x.repeat(2)),
+    _state("step", lambda x: x.to(torch.complex64)), _state("step", lambda x: x * float("nan")),
+    _state("exp_avg", lambda x: x[:-1]), _state("exp_avg", lambda x: x.double()), _state("exp_avg", lambda x: None), _state("exp_avg", _between),
+    _state("exp_avg_sq", lambda x: x.cpu()), _state("exp_avg_sq", lambda x: torch.nn.Parameter(x)),
+])
+def test_both_hosts_take_the_same_slices(cuda_lib, monkeypatch, change):
+    opt = _stepped(False)
+    change(opt, monkeypatch)
+    native = opt._adamw_updates() is not None
+    monkeypatch.setattr(zero, "_native", ())
+    assert (opt._adamw_updates() is not None) == native
+
+
 @pytest.mark.gpu
 def test_optimizers_dtypes_and_surroundings_the_kernel_does_not_take(cuda_lib, monkeypatch):
     assert _stepped(False, cls=torch.optim.Adam)._adamw_updates() is None
