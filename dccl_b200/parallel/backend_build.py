@@ -3,7 +3,8 @@ libdccl.so, and loads it.
 
 The extension only uses the library's public C++ API and libtorch; it is compiled with the system
 C++ compiler against the headers of the installed torch and linked to ``dccl_b200/lib/libdccl.so``
-by relative rpath, so the built file can be moved with the package.
+by relative rpath, so the built file can be moved with the package. Its name carries the versions of torch and of Python whose
+inline code it holds: after either is replaced, it is a missing file and not one that reads objects of another layout.
 """
 import importlib.util
 import os
@@ -12,12 +13,14 @@ import subprocess
 import sys
 import sysconfig
 
+import torch
+
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _PKG = os.path.dirname(_HERE)
 _ROOT = os.path.dirname(_PKG)
 SRC_DIR = os.path.join(_ROOT, "csrc", "torch")
 SRCS = [os.path.join(SRC_DIR, name) for name in ("pg_dccl.cpp", "adamw_step.cpp")]
-OUT = os.path.join(_PKG, "lib", "_dccl_torch.so")
+OUT = os.path.join(_PKG, "lib", "_dccl_torch-%s-torch%s.so" % (sys.implementation.cache_tag, torch.__version__))
 
 
 def needs_build():
@@ -31,7 +34,6 @@ def needs_build():
 def build(force=False, verbose=False):
     if not force and not needs_build():
         return OUT
-    import torch
     from torch.utils import cpp_extension
     from .._lib import LIB_PATH, lib
     lib()   # makes sure libdccl.so exists

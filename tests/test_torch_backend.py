@@ -1,11 +1,13 @@
 """torch.distributed backend "dccl": every collective against values computed from the ranks' seeds,
 DistributedDataParallel gradients against a serial reference. CPU tensors here; CUDA tensors in the
 gpu-marked tests."""
+import importlib.util
 import os
 
 import pytest
 
 from conftest import gpu_count
+from dccl_b200.parallel import backend_build
 from dccl_b200.utils.launch import python_ranks
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -17,6 +19,18 @@ def run(world, args, gpus=False, timeout=600):
     for r, p in enumerate(res):
         assert p.returncode == 0, "rank %d:\n%s\n%s" % (r, p.stdout[-2000:], p.stderr[-3000:])
         assert p.stdout.strip().endswith("OK")
+
+
+def test_an_extension_of_another_torch_is_not_loaded(monkeypatch):
+    backend_build.build()
+    assert not backend_build.needs_build()
+    monkeypatch.setattr(backend_build.torch, "__version__", "1.0.0")
+    spec = importlib.util.spec_from_file_location("backend_build_of_another_torch", backend_build.__file__)
+    other = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(other)
+    assert other.needs_build()
+    with pytest.raises(ImportError):
+        other.load()
 
 
 @pytest.mark.parametrize("world", [2, 4])
