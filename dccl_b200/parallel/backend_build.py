@@ -6,6 +6,7 @@ C++ compiler against the headers of the installed torch and linked to ``dccl_b20
 by relative rpath, so the built file can be moved with the package. Its name carries the versions of torch and of Python whose
 inline code it holds: after either is replaced, it is a missing file and not one that reads objects of another layout.
 """
+import fcntl
 import importlib.util
 import os
 import shutil
@@ -32,8 +33,18 @@ def needs_build():
 
 
 def build(force=False, verbose=False):
+    """Compiles the extension unless it is up to date. Of several ranks one compiles and the others wait for its file."""
     if not force and not needs_build():
         return OUT
+    os.makedirs(os.path.dirname(OUT), exist_ok=True)
+    with open(OUT + ".lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)        # given back by the system when its holders have ended: this process and the compiler
+        if force or needs_build():
+            _compile(lock, verbose)
+    return OUT
+
+
+def _compile(lock, verbose):
     from torch.utils import cpp_extension
     from .._lib import LIB_PATH, lib
     lib()   # makes sure libdccl.so exists
@@ -42,21 +53,19 @@ def build(force=False, verbose=False):
     tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
     incs = cpp_extension.include_paths(device_type="cuda")
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    part = "%s.%d" % (OUT, os.getpid())      # ranks that build at the same time do not write into each other's file
+    part = OUT + ".part"                        # one name: what a killed compiler left is written over by the next
     cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", *SRCS, "-o", part,
            "-DTORCH_EXTENSION_NAME=_dccl_torch", "-DTORCH_API_INCLUDE_EXTENSION_H", "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
            "-I" + os.path.join(_ROOT, "include"), "-I" + os.path.join(cuda_home, "include"), "-I" + sysconfig.get_paths()["include"]]
     cmd += ["-I" + p for p in incs]
     cmd += ["-L" + tlib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
             "-L" + os.path.dirname(LIB_PATH), "-ldccl", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + tlib, "-Wno-attributes", "-Wno-interference-size"]
-    os.makedirs(os.path.dirname(OUT), exist_ok=True)
-    res = subprocess.run(cmd, capture_output=True, text=True)
+    res = subprocess.run(cmd, capture_output=True, text=True, pass_fds=(lock.fileno(),))
     if res.returncode != 0:
         raise RuntimeError("building the torch backend failed:\n" + " ".join(cmd) + "\n" + res.stderr[-6000:])
     os.replace(part, OUT)
     if verbose:
         print(res.stderr, file=sys.stderr)
-    return OUT
 
 
 _module = None

@@ -3,6 +3,10 @@ DistributedDataParallel gradients against a serial reference. CPU tensors here; 
 gpu-marked tests."""
 import importlib.util
 import os
+import subprocess
+import threading
+import time
+from concurrent.futures import ThreadPoolExecutor
 
 import pytest
 
@@ -31,6 +35,39 @@ def test_an_extension_of_another_torch_is_not_loaded(monkeypatch):
     assert other.needs_build()
     with pytest.raises(ImportError):
         other.load()
+
+
+@pytest.mark.parametrize("force", [False, True])
+def test_ranks_that_find_no_extension_compile_it_one_at_a_time(monkeypatch, tmp_path, force):
+    out, running, compiled = str(tmp_path / "lib" / "extension.so"), threading.Lock(), []
+
+    def compiler(cmd, **kw):
+        assert running.acquire(blocking=False), "two compilers at a time"
+        time.sleep(0.2)
+        path = cmd[cmd.index("-o") + 1]
+        with open(path, "w") as f:
+            f.write("complete")
+        compiled.append(path)
+        running.release()
+        return subprocess.CompletedProcess(cmd, 0, "", "")
+
+    monkeypatch.setattr(backend_build, "OUT", out)
+    monkeypatch.setattr(backend_build.subprocess, "run", compiler)
+    with ThreadPoolExecutor(4) as ranks:
+        assert [f.result() for f in [ranks.submit(backend_build.build, force) for _ in range(4)]] == [out] * 4
+    assert len(compiled) == (4 if force else 1) and out not in compiled
+    assert open(out).read() == "complete" and not [p for p in compiled if os.path.exists(p)]
+
+
+def test_what_a_killed_compiler_leaves_does_not_pile_up(monkeypatch, tmp_path):
+    monkeypatch.setattr(backend_build, "OUT", str(tmp_path / "extension.so"))
+    left = set()
+    for pid in (11, 12, 13):
+        monkeypatch.setattr(backend_build.os, "getpid", lambda: pid)
+        monkeypatch.setattr(backend_build.subprocess, "run", lambda cmd, **kw: (left.add(cmd[cmd.index("-o") + 1]), 1 / 0))
+        with pytest.raises(ZeroDivisionError):
+            backend_build.build()
+    assert len(left) == 1
 
 
 @pytest.mark.parametrize("world", [2, 4])
