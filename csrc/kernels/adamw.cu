@@ -3,6 +3,7 @@
  * between the reduce-scatter and the all-gather of dccl_b200/parallel/zero.py. Masters and moments are fp32; the gradient
  * arrives and the updated parameters leave in the parameters' own type.
  */
+#include "adamw.hpp"
 #include "launch_early.cuh"
 #include "../device/reduce_ops.cuh"
 #include <cstdint>
@@ -87,10 +88,6 @@ __global__ void __launch_bounds__(kAdamWThreads) k_adamw(const __grid_constant__
 
 using namespace dccl;
 
-/**
- * AdamW on `n` elements that live on `device`: master, moments and out are updated, master_grad receives the gradient in
- * fp32. dtype: ncclDataType_t of grad and out (float16, float32 or bfloat16). Returns 0, or -1 after a message on stderr.
- */
 extern "C" int dccl_adamw_flat(int device, int dtype, size_t n, void* master, void* master_grad, void* m, void* v, const void* grad, void* out,
                                double decay, double w1, double b2, double w2, double step, double bc2_sqrt, double eps, void* stream_v) {
     if (!n) return 0;

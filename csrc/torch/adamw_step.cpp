@@ -6,6 +6,7 @@
  * Plain CPython functions: their arguments are borrowed and not converted. Everything that could throw is caught at this border.
  */
 #include "adamw_step.hpp"
+#include "../kernels/adamw.hpp"
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/object_ptr.h>
@@ -16,8 +17,7 @@
 
 namespace {
 
-using FlatUpdate = int (*)(int device, int dtype, size_t n, void* master, void* master_grad, void* m, void* v, const void* grad, void* out,
-                           double decay, double w1, double b2, double w2, double step, double bc2_sqrt, double eps, void* stream);
+using FlatUpdate = decltype(&dccl_adamw_flat);
 
 /** ncclDataType_t of the parameters' types that the kernel takes, or -1. */
 int flat_dtype(at::ScalarType t) { return t == at::kHalf ? 6 : t == at::kFloat ? 7 : t == at::kBFloat16 ? 9 : -1; }

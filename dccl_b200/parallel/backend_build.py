@@ -21,15 +21,15 @@ _PKG = os.path.dirname(_HERE)
 _ROOT = os.path.dirname(_PKG)
 SRC_DIR = os.path.join(_ROOT, "csrc", "torch")
 SRCS = [os.path.join(SRC_DIR, name) for name in ("pg_dccl.cpp", "adamw_step.cpp")]
+HEADERS = [os.path.join(SRC_DIR, "adamw_step.hpp"), os.path.join(_ROOT, "csrc", "kernels", "adamw.hpp"), os.path.join(_ROOT, "include", "dccl", "dccl.hpp")]
 OUT = os.path.join(_PKG, "lib", "_dccl_torch-%s-torch%s.so" % (sys.implementation.cache_tag, torch.__version__))
 
 
 def needs_build():
     if not os.path.exists(OUT):
         return True
-    sources = SRCS + [os.path.join(SRC_DIR, "adamw_step.hpp"), os.path.join(_ROOT, "include", "dccl", "dccl.hpp")]
     # a package that came without its sources is as new as it gets
-    return any(os.path.exists(f) and os.path.getmtime(OUT) < os.path.getmtime(f) for f in sources)
+    return any(os.path.exists(f) and os.path.getmtime(OUT) < os.path.getmtime(f) for f in SRCS + HEADERS)
 
 
 def build(force=False, verbose=False):

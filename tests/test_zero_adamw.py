@@ -1,7 +1,10 @@
 """The one-kernel AdamW update of dccl_b200.parallel.zero against the general path (torch's own optimizer and the casts
 around it), and which optimizers may take it."""
 import collections
+import ctypes
 import functools
+import os
+import re
 import warnings
 
 import numpy as np
@@ -452,6 +455,23 @@ def test_options_that_python_takes_for_others(cuda_lib, monkeypatch, name, value
     opt = _stepped(False)
     _option(name, lambda: value)(opt, monkeypatch)
     assert opt._adamw_updates() is None
+
+
+def test_the_entry_point_is_declared_once(dccl_lib, monkeypatch):
+    """By the header: the extension, which calls it by address, is older than a changed one, and ctypes has the same arguments."""
+    if not hasattr(dccl_lib, "dccl_adamw_flat"):
+        pytest.skip("a host-only library")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    header = os.path.join(root, "csrc", "kernels", "adamw.hpp")
+    kinds = {"int": ctypes.c_int, "size_t": ctypes.c_size_t, "double": ctypes.c_double}
+    arguments = re.search(r"int dccl_adamw_flat\((.*?)\);", open(header).read(), re.S).group(1).split(",")
+    assert dccl_lib.dccl_adamw_flat.argtypes == [ctypes.c_void_p if "*" in a else kinds[a.split()[0]] for a in arguments]
+    for name in ("kernels/adamw.cu", "torch/adamw_step.cpp"):
+        assert "adamw.hpp\"" in open(os.path.join(root, "csrc", name)).read()
+    zero.backend_build.build()
+    stock = os.path.getmtime
+    monkeypatch.setattr(os.path, "getmtime", lambda f: 1e12 if os.path.realpath(f) == os.path.realpath(header) else stock(f))
+    assert zero.backend_build.needs_build()
 
 
 def test_the_extension_is_loaded_without_a_compiler_or_not_at_all(monkeypatch, tmp_path):
