@@ -10,12 +10,12 @@
 namespace dccl {
 
 /** Sum, maximum and minimum of one-byte integers; a product needs more than its byte in between. */
-template <typename T, int OP> constexpr bool kFoldsBytes = sizeof(T) == 1 && OP != OP_PROD;
+template <typename T, int OP> constexpr bool kFoldsBytes = (std::is_same<T, int8_t>::value || std::is_same<T, uint8_t>::value) && OP != OP_PROD;
 
 /** Sum, maximum and minimum of TWO 16-bit floats: the sum of more is kept in fp32 in between. Of two, the packed addition rounds
  *  as an fp32 sum does that is rounded to the type after it (fp32 has more than twice its digits, and two more), so the
  *  bits are the same; a product of bf16 can be so small that they are not. */
-template <typename T, int OP> constexpr bool kFoldsPairs = sizeof(T) == 2 && OP != OP_PROD;
+template <typename T, int OP> constexpr bool kFoldsPairs = (std::is_same<T, __half>::value || std::is_same<T, __nv_bfloat16>::value) && OP != OP_PROD;
 
 template <typename T, int OP> __device__ __forceinline__ uint32_t fold_packed(uint32_t x, uint32_t y) {
     if constexpr (kFoldsPairs<T, OP>) {
