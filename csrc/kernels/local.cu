@@ -6,6 +6,7 @@
 #include "packed_ops.cuh"
 #include "launch_early.cuh"
 #include "kernels.hpp"
+#include "local_shapes.hpp"
 #include "../device/reduce_ops.cuh"
 
 namespace dccl {
@@ -131,22 +132,10 @@ __global__ void __launch_bounds__(THREADS) k_local_reduce(T* acc, const T* in, c
 cudaError_t launch_local_copy(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
     if (!bytes || dst == src) return cudaSuccess;
     const Cut c = cut_range(dst, src, bytes);
-    // CTAs of 1024 threads once a copy streams out of HBM, of 256 before: probe of the two, us, 20 MiB 7.46 / 7.18, 24 MiB
-    // 8.74 / 8.73, 28 MiB 9.99 / 10.15, 32 MiB 11.18 / 11.35, 64 MiB 20.82 / 21.07, 1 GiB 305 / 309; 25 MiB from a source 6
-    // bytes off 9.52 / 9.40
-    const unsigned threads = bytes >= (28u << 20) ? 1024 : 256;
+    const unsigned threads = copy_threads(bytes);
     const size_t per = (size_t)threads * kCopyU, grid = (c.nv + per - 1) / per;
     return launch_early(threads == 1024 ? k_local_copy<1024> : k_local_copy<256>, (unsigned)(grid ? grid : 1), threads, stream, (char*)dst, (const char*)src, c);
 }
-
-/**
- * The shape of a fold of `bytes` per operand. One vector per thread and CTAs of 512 stream best out of HBM; where both operands
- * can be in L2, its latency counts and two vectors per thread in CTAs of 128 are ahead. Probe of the two shapes, us, operands
- * of three sets in turn / of sets that come from HBM: 8 MiB 2.75 -> 2.63 / 4.63 -> 4.79, 12 MiB 3.71 -> 3.62 / 6.33 -> 6.14,
- * 16 MiB 6.95 -> 6.15 / 8.51 -> 8.51, 20 MiB 10.21 -> 9.40 / 10.57 -> 10.55, 22 MiB 11.19 -> 10.61 / 11.45 -> 11.54,
- * 24 MiB 12.21 -> 12.02 / 12.30 -> 12.44, 28 MiB 14.00 -> 14.16 / 13.97 -> 14.15, 1 GiB 450 -> 457.
- */
-static bool two_vectors(size_t bytes) { return bytes >= (10u << 20) && bytes <= (22u << 20); }
 
 cudaError_t launch_local_reduce(void* acc, const void* in, size_t count, ncclDataType_t dt, ncclRedOp_t op, cudaStream_t stream) {
     if (!count) return cudaSuccess;

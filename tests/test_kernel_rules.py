@@ -26,3 +26,26 @@ def test_types_that_fold_several_elements_at_a_time(tmp_path):
     res = subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I" + ROOT, "-I" + os.path.join(ROOT, "include"), "-DDCCL_WITH_CUDA_RUNTIME",
                           "-c", str(tmp_path / "types.cu"), "-o", str(tmp_path / "types.o")], capture_output=True, text=True)
     assert res.returncode == 0, res.stderr[-2000:]
+
+
+SHAPES = """
+#include "csrc/kernels/local_shapes.hpp"
+constexpr size_t kL2 = 126000000;
+constexpr bool copies_out_of_l2_in_small_ctas() {
+    for (size_t bytes = 4096; 2 * bytes <= kL2; bytes += 4096)
+        if (dccl::copy_threads(bytes) != 256) return false;
+    return true;
+}
+static_assert(copies_out_of_l2_in_small_ctas(), "a pair of buffers that fits into L2");
+static_assert(dccl::copy_threads(kL2) == 1024 && dccl::copy_threads(size_t(1) << 30) == 1024 && dccl::copy_threads(size_t(1) << 40) == 1024, "a pair that does not");
+"""
+
+
+# A pair of buffers that fits into L2 is copied from there when it comes again, 6 to 12 % slower in CTAs of 1024.
+def test_copies_that_can_come_out_of_l2_keep_their_shape(tmp_path):
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if not cxx:
+        pytest.skip("needs a C++ compiler")
+    (tmp_path / "shapes.cpp").write_text(SHAPES)
+    res = subprocess.run([cxx, "-std=c++17", "-fsyntax-only", "-fconstexpr-loop-limit=1000000", "-I" + ROOT, str(tmp_path / "shapes.cpp")], capture_output=True, text=True)
+    assert res.returncode == 0, res.stderr[-2000:]

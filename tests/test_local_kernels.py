@@ -38,6 +38,11 @@ def test_copy_at_every_pair_of_offsets(comm, nbytes):
             assert torch.equal(dst, want), (nbytes, so, do)
 
 
+@pytest.mark.parametrize("nbytes", [(80 << 20) - 1, 80 << 20, (80 << 20) + 32768 + 17])
+def test_copy_where_its_ctas_grow(comm, nbytes):
+    test_copy_where_its_shape_changes(comm, nbytes)
+
+
 @pytest.mark.parametrize("nbytes", [(28 << 20) - 1, 28 << 20, (28 << 20) + 32768 + 17])
 def test_copy_where_its_shape_changes(comm, nbytes):
     src = torch.randint(0, 255, (nbytes + 32,), dtype=torch.uint8, device="cuda", generator=torch.Generator(device="cuda").manual_seed(nbytes))
