@@ -82,9 +82,9 @@ bool counts_in_place(PyObject* count, const at::Tensor& t) {
 
 /** A step count of zero or more. Below zero the bias corrections divide by zero or have no square root, which torch's step reports. */
 bool counts_up(PyObject* count) {
-    const at::Tensor t = THPVariable_Unpack(count);
-    if (t.numel() != 1 || t.is_complex()) return false;
-    return (counts_in_place(count, t) ? (double)*t.const_data_ptr<float>() : t.item().toDouble()) >= 0;
+    if (counts_in_place(count, THPVariable_Unpack(count))) return *THPVariable_Unpack(count).const_data_ptr<float>() >= 0;
+    const at::Tensor t = THPVariable_Unpack(count);        // a copy: item() can run Python
+    return t.numel() == 1 && !t.is_complex() && t.item().toDouble() >= 0;
 }
 
 /** adamw_ready(param_group, state, master, master_grad, grad, n): whether the kernel can update this slice of n elements, now that
