@@ -9,6 +9,8 @@ ncu capture: inputs larger than L2, a few GB on the device at most, two launches
     python benchmarks/profile_emu.py --kind sendrecv --ranks 8 --mb 64 --ctas 16                          (k_p2p, ring of pairs)
     python benchmarks/profile_emu.py --kind sendrecv --ranks 8 --mb 64 --ctas 16 --rendezvous             (k_p2p, direct stores into the receive buffers)
     python benchmarks/profile_emu.py --kind local_reduce --mb 256                                         (k_local_reduce, one rank)
+    python benchmarks/profile_emu.py --kind local_fold --mb 16                                            (k_local_reduce, bf16 at odd elements)
+    python benchmarks/profile_emu.py --kind local_copy --mb 512                                           (k_local_copy, one-rank all-reduce of bf16)
     python benchmarks/profile_emu.py --kind switch --mb 256 --ctas 16     (k_nvls on a one-member multicast object, where the driver allows one)
     ncu --set full --clock-control none -k regex:k_twoshot -c 1 -o prof_twoshot \\
         python benchmarks/profile_emu.py --kind allreduce --algo twoshot --ranks 8 --mb 64 --ctas 16
@@ -22,6 +24,27 @@ import numpy as np
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT)
 from dccl_b200._lib import lib  # noqa: E402
+
+
+def one_gpu_call(args, L):
+    """The copy or the fold on device buffers, in bf16; True when the result is right."""
+    import torch
+    from dccl_b200 import Communicator
+    from dccl_b200.comm import OPS, dtype_of
+    count = int(args.mb * (1 << 20)) // 2
+    a, b = (torch.full((count + 3,), v, dtype=torch.bfloat16, device="cuda") for v in (0.0, 1.0))
+    if args.kind == "local_copy":
+        comm = Communicator(rank=0, world=1, device=0)
+        for _ in range(args.iters):
+            comm.all_reduce(b[:count], a[:count])
+        torch.cuda.synchronize()
+        comm.finalize()
+        return bool((a[:count] == 1.0).all())
+    for _ in range(args.iters):
+        rc = L.dccl_local_reduce_device(a[1:].data_ptr(), b[3:].data_ptr(), count, dtype_of(a), OPS["sum"], torch.cuda.current_stream().cuda_stream)
+        if rc != 0:
+            return False
+    return bool((a[1:1 + count] == float(args.iters)).all()) and float(a[0]) == 0.0
 
 
 def main():
@@ -47,6 +70,8 @@ def main():
         rc = L.dccl_emu_switch_single(7, 0, count, args.ctas, args.iters, hin.ctypes.data, hout.ctypes.data)
         print("rc", rc, "(-10: no multicast here, -11: set-up refused)", "match", bool(rc == 0 and np.array_equal(hin, hout)))
         sys.exit(0 if rc == 0 and np.array_equal(hin, hout) else 1)
+    if args.kind in ("local_copy", "local_fold"):
+        sys.exit(0 if one_gpu_call(args, L) else 1)
     if args.kind == "local_reduce":
         count = int(args.mb * (1 << 20)) // 4
         a = np.ones(count, dtype=np.float32)

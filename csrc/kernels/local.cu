@@ -60,7 +60,7 @@ static Cut cut_range(const void* dst, const void* src, size_t bytes) {
 
 /**
  * HBM bounds a large copy, launch and latency a small one. Every thread moves two vectors and the CTAs follow each other
- * through memory, so that all SMs work in one window of a few MB: 1 GiB takes 304 us (7.1 TB/s of reads and writes) where
+ * through memory, so that all SMs work in one window of a few MB: 1 GiB takes 305 us (7.0 TB/s of reads and writes) where
  * two resident CTAs per SM, each on a contiguous piece of its own, took 363 us (296 places of memory open at once). Pointers
  * with different distances to a 16-byte boundary cost a second load, which the L1 cache serves, and a few selects: 26 MB of
  * bf16 from a source 6 bytes off take 9.4 us where a loop over single bytes took 88.2 us.
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(THREADS) k_local_copy(char* dst, const char* s
 
 /**
  * acc[i] = op(acc[i], in[i]): three streams of HBM traffic and nothing else, the CTAs following each other through memory as in
- * the copy: 1 GiB fp32 takes 446 us (7.2 TB/s), 25 MiB bf16 12.7 us and 1 MiB 3.3 us (the host's cost of the call), where two
+ * the copy: 1 GiB fp32 takes 448 us (7.2 TB/s), 25 MiB bf16 12.7 us and 1 MiB 3.3 us (the host's cost of the call), where two
  * resident CTAs per SM with eight vectors in flight per thread, each CTA on a piece of at least 64 KB, took 520, 16.4 and 5.1 us.
  * Operands at different distances from a 16-byte boundary read `in` through a window as the copy does: 12 MB of fp16 24.6 ->
  * 3.9 us (before: one element per access). The elements outside the vectors get threads of their own behind the vectors' threads.

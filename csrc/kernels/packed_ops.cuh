@@ -1,8 +1,8 @@
 /**
  * Four one-byte elements or two 16-bit floats in one operation, where elements unpacked one by one cost more instructions than
  * a streaming kernel hides. Folding 256 MB of bytes for maximum or minimum took 141 us for int8 and 123 us for uint8 where every
- * other type takes 113; now these do, too. 16-bit floats cost up to eleven instructions for a pair, which shows where the operands
- * are in L2: the maximum of 12 MB of fp16 at odd elements 4.34 -> 3.86 us, the sum of 16 MiB of bf16 6.30 -> 6.19.
+ * other type takes 113; now these do, too. Of 16-bit floats it shows where the operands are in L2: the
+ * maximum of 12 MB of fp16 at odd elements 4.34 -> 3.86 us, the sum of 16 MiB of bf16 6.30 -> 6.19.
  */
 #pragma once
 #include "../device/reduce_ops.cuh"

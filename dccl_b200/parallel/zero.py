@@ -231,7 +231,7 @@ class ShardedOptimizer:
     def _adamw_range(self, updates):
         """The updates, where torch's optimizers show their step: inside the range that the profiler and other observers know
         it by, with the call at its end through which the profiler finds the optimizer. An unobserved range costs a step
-        2.4 us of 15.8 and is left out."""
+        2.0 us on top of 5.6 and is left out."""
         entered = _enter_range("Optimizer.step#AdamW.step") if _observed() else None
         try:
             for u in updates:
